@@ -18,13 +18,13 @@ __device__ __forceinline__ int expert_of_row(const int *offsets, int E, int r) {
   return lo;
 }
 
-// dot of one weight row (packed codes inside the 16 KB weight tiles: `codes` points at the row's 64 bytes in the
-// first tile of its row block, the next 128 k follow one tile further; raw row-major scales) with an fp16 row
+// dot of one weight row (packed codes inside the weight tiles: `codes` points at the row's 64 bytes in the first
+// tile of its 120 rows; raw row-major scales) with an fp16 row
 __device__ __forceinline__ float warp_dot_mxfp4(const uint8_t *codes, const uint8_t *scales, const __half *x,
                                                 int K, int lane) {
   float acc = 0.f;
   for (int b = lane; b < K / 32; b += 32) {
-    const uint4 c = *reinterpret_cast<const uint4 *>(codes + static_cast<size_t>(b >> 2) * kWTileStride + (b & 3) * 16);
+    const uint4 c = *reinterpret_cast<const uint4 *>(codes + w_codes_offset(b >> 2) + (b & 3) * 16);
     uint32_t w[16];
     sm100::dequant_block32(c, sm100::e8m0_to_f16x2(scales[b]), w);
     const uint4 *xp = reinterpret_cast<const uint4 *>(x + b * 32);
@@ -46,10 +46,10 @@ __device__ __forceinline__ float warp_dot_mxfp4(const uint8_t *codes, const uint
   return acc;
 }
 
-// the 64 code bytes of row `row` of expert e's [R x K] matrix in the first tile of the row's block
+// the 64 code bytes of row `row` of expert e's [R x K] matrix in the first tile of the row's 120
 __device__ __forceinline__ const uint8_t *tile_row(const uint8_t *w_tiles, int e, int row, int R, int K) {
-  const int n_nt = (R + kTileN - 1) / kTileN, n_kc = (K + kChunkK - 1) / kChunkK;
-  return w_tiles + (static_cast<size_t>(e) * n_nt + row / kTileN) * n_kc * kWTileStride + (row % kTileN) * (kChunkK / 2);
+  const int n_half = 2 * ((R + kBlockRows - 1) / kBlockRows), n_kc = (K + kChunkK - 1) / kChunkK;
+  return w_tiles + (static_cast<size_t>(e) * n_half + row / kHalfRows) * n_kc * kWTileBytes + (row % kHalfRows) * (kChunkK / 2);
 }
 
 __global__ void __launch_bounds__(256)

@@ -10,31 +10,41 @@
 // go from HBM through TMA straight into the tensor core; no thread touches a
 // weight.
 //
-// Why this shape.  Issuing a tcgen05.mma costs its thread ~47 cycles whatever its
-// shape, a wait or a commit more than that, and the block-scaled kinds exist for
-// M = 128 only, so what counts is MACs per instruction and per pipeline step:
-// weights go on the N axis (240 rows per work item; 240 divides both 5760 and
-// 2880 and leaves tensor memory for two accumulators) and the tokens of one
-// expert on the M = 128 axis.  There is no
-// bf16 x fp4 instruction, so every bf16 activation is split into two e4m3 terms
-// (high + low, exact for bf16 inputs): a token tile is 64 tokens = 128 rows,
-// row 2i the high term of token i, row 2i+1 its low term whose block scale
-// carries the extra 2^-4.  The two partial sums land in adjacent lanes of the
-// accumulator and are added in the epilogue.
+// There is no bf16 x fp4 instruction, so every bf16 activation is split into two e4m3
+// terms (high + low, exact for bf16 inputs): row 2i of a token tile is the high term of its
+// token i, row 2i+1 the low term, whose block scale carries the extra 2^-4.  The two partial
+// sums land in adjacent columns of the accumulator and are added in the epilogue.
 //
-// Per 128-element slice of k (one shared-memory stage) the producer warp
-// issues: weight codes [240 rows x 128] (TMA, 16U4_ALIGN16B: 4-bit codes are
-// expanded to the 8-bit containers the MMA reads, 128-byte swizzle), weight
-// scales (two 512-byte atoms, pre-tiled at load time), activations [128 rows x
-// 128] e4m3 (TMA, 128-byte swizzle).  The MMA warp copies the scale atoms to
-// tensor memory (tcgen05.cp) and issues four K = 32 instructions.  Both warps
-// stay converged and elect one lane per instruction group, so that descriptors
-// and tensor-memory addresses live in uniform registers.  Sixteen epilogue
-// warps drain the fp32 accumulator (double buffered: 2 x 240 columns).
-// What bounds the kernel is the SM's shared-memory port (128 bytes per cycle,
-// shared by the copy engine's writes and the tensor core's reads): an M128 N240
-// K32 instruction moves 23.5 KB through it, 184 cycles against 120 of tensor pipe.
-// No cluster launch, no multicast: every CTA fetches its own tiles.
+// Why this shape.  Two CTAs (a cluster, one TPC) work on one item: 240 weight rows
+// against up to 96 tokens of one expert, M256 (120 of 128 rows used in each CTA; 240 divides
+// both 5760 and 2880) x N x K32 instructions of cta_group::2.  The weights are the M operand,
+// so that N follows the number of tokens in steps of 8 and an expert with a few rows pays for
+// a few rows; each CTA holds its own 120 weight rows and HALF of the token rows, which its
+// tensor core shares with the peer's, so the token tile crosses L2 -> SM and the shared-memory
+// port once per pair.
+//
+// Per 128-element slice of k (two to a shared-memory stage) each CTA loads: weight codes
+// [120 rows x 128] (TMA, 16U4_ALIGN16B: 4-bit codes are expanded to the 8-bit containers the
+// MMA reads, 128-byte swizzle), their 512-byte scale atom (pre-tiled at load time), and its
+// half of the token rows.  The weights of both slices are one TMA box, the token rows one plain bulk
+// copy (the quantiser and the SwiGLU epilogue write them interleaved by slice and with the 128-byte
+// swizzle already applied): what a role spends per stage is issue time, ~150 cycles per copy, ~110
+// per wait, ~35 per commit, and it was that time that bounded earlier forms with one slice per stage.
+// Two producer warps (weights and their scales; tokens) keep kStages stages in flight.  The MMA warp
+// of the even CTA copies the scales of both CTAs to tensor memory (tcgen05.cp) and issues four
+// instructions per slice for the pair; the
+// same warp of the odd CTA reports each stage that has landed in its shared memory to the even
+// one.  Issuing warps stay converged and elect one lane, so that descriptors and
+// tensor-memory addresses live in uniform registers.  Sixteen epilogue warps per CTA drain the
+// fp32 accumulator (double buffered: 2 x 192 columns).
+// One more warp counts finished MLP1 items for the MLP2 items that wait for them.
+// No multicast: every CTA fetches its own tiles.
+//
+// Measured (B200, one launch of both phases, us, layer of 128 experts, hidden and
+// intermediate size 2880; before: one CTA per item of 64 tokens x 240 rows, tokens on the fixed M = 128 axis): 32 rows 179 -> 174,
+// 256 rows 324 -> 299, 1856 rows 412 -> 396, 8192 rows 1459 -> 1403.  Alone at 256 rows the copies take 269 (HBM at its
+// peak) and the MMAs 214: what is left is the round trip of the ring.  At 8192 rows the tensor pipe is busy 87 % of
+// the cycles and the power cap sets the clock (1.29 GHz).
 #include <cuda_fp8.h>
 
 #include "moe_internal.cuh"
@@ -46,191 +56,249 @@ namespace moe {
 using namespace sm100;
 
 constexpr int kStages = 4;
-constexpr int kABytes = kTileM * kChunkK;         // 16384: 128 rows x 128 e4m3
-constexpr int kWBytes = kTileNPad * kChunkK;      // 32768: 256 rows x 128 containers (240 loaded)
-// the transaction count of a 16U4_ALIGN16B copy is the PACKED size: 240 rows x 64 bytes
-constexpr int kWLoadBytes = kTileN * kChunkK / 2; // 15360
-constexpr int kStageBytes = kABytes + kWBytes + kSfbChunkBytes;  // 50176
-constexpr int kSfaSlots = 4;                      // per-item activation scale atoms, a ring of their own
-constexpr int kSfaOff = kStages * kStageBytes;
-constexpr int kBarOff = kSfaOff + kSfaSlots * kSfAtomBytes;
-constexpr int kNumBars = 2 * kStages + 4 + 2 * kSfaSlots;  // full, empty, d_full[2], d_empty[2], sfa_full, sfa_empty
-constexpr int kSmemBytes = kBarOff + 8 * kNumBars + 16 + 1024 /*alignment slack*/;
+constexpr int kSlices = 2;                        // k slices per stage: one wait and one commit for eight MMAs
+constexpr int kWBytes = kHalfRows * kChunkK;      // 15360: 120 rows x 128 containers
+// the transaction count of a 16U4_ALIGN16B copy is the PACKED size: 120 rows x 64 bytes
+constexpr int kWLoadBytes = kWTileCodes;
+// the M = 128 rows of a weight slice are read 8 rows into what follows it: rows 120..127 of the accumulator are
+// never used
+constexpr int kXOff = kSlices * kWBytes;
+constexpr int kSfaOff = kXOff + kPairBytes / 2;             // 24576: this CTA's half of the token rows, at most
+constexpr int kSfbOff = kSfaOff + kSlices * kSfAtomBytes;   // token scales, loaded with the first stage of an item
+constexpr int kStageBytes = kSfbOff + kSfbTileBytes;        // 57344
+constexpr int kBarOff = kStages * kStageBytes;
+constexpr int kNumBars = 2 * kStages + 4;         // full, empty, d_full[2], d_empty[2]
+constexpr int kProgOff = kBarOff + 8 * kNumBars + 16;       // MLP1 items finished by each epilogue warp
+constexpr int kSmemBytes = kProgOff + 16 * 4 + 1024 /*alignment slack*/;
 
 constexpr int kEpiWarps = 16;             // four per tensor-memory lane quadrant
-constexpr int kEpiChunks = 4;             // 16-column chunks per epilogue warp (15 in all)
-constexpr int kProducerWarp = 16, kMmaWarp = 17;
-constexpr int kThreads = 18 * 32;
+constexpr int kWProducerWarp = 16, kXProducerWarp = 17, kMmaWarp = 18, kDoneWarp = 19;
+constexpr int kThreads = 20 * 32;
 
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kAccBufCols = kTileN;          // accumulator buffer d at columns d*240
-constexpr uint32_t kSfaCol0 = 480;                // + 4*(item & 1)
-constexpr uint32_t kSfbCol0 = 488;                // + 8*(chunk & 1)
+constexpr uint32_t kAccBufCols = kTileRows;       // accumulator buffer d at columns d*192
+constexpr uint32_t kSfbCol0 = 2 * kAccBufCols;    // + 8*(item & 1): token scales
+constexpr uint32_t kSfaCol0 = kSfbCol0 + 16;      // + 4*(slice & 3): weight scales
 
-static_assert(kStageBytes % 1024 == 0, "stages must keep 1024-byte alignment for the swizzled tiles");
+static_assert(kSfaCol0 + 16 <= kTmemCols, "tensor memory");
+static_assert(kWBytes % 1024 == 0 && kPairBytes % 2048 == 0 && kStageBytes % 1024 == 0, "swizzled tiles keep 1024-byte alignment");
 static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
 
-__device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float d) {
-  const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
-  const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E4M3);
-  return lo | (hi << 16);
+// Two fp32 values -> two e4m3 bytes (first value in the low byte), and back.
+__device__ __forceinline__ uint32_t pack_e4m3x2(float a, float b) {
+  return __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
 }
-__device__ __forceinline__ float e4m3_to_float(uint32_t byte) {
-  const __half_raw h = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>(byte), __NV_E4M3);
-  return __half2float(*reinterpret_cast<const __half *>(&h));
+__device__ __forceinline__ float2 unpack_e4m3x2(uint32_t v) {
+  const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(v), __NV_E4M3);
+  return __half22float2(__half2(h));
 }
 
+__device__ __forceinline__ void st_release_cta(uint32_t saddr, uint32_t v) {
+  asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(saddr), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t ld_acquire_cta(uint32_t saddr) {
+  uint32_t v;
+  asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(saddr) : "memory");
+  return v;
+}
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const unsigned int *p) {
   uint32_t v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 
+// 4 x 4 byte transposes of two words across the four lanes that differ in bits 1 and 2: before, lane q holds four
+// tokens of feature q, afterwards four features of token q.
+__device__ __forceinline__ void transpose_pair(uint32_t &w0, uint32_t &w1, int q) {
+  const bool b1 = (q & 2) != 0, b0 = (q & 1) != 0;
+  uint32_t r = __shfl_xor_sync(0xffffffffu, __byte_perm(w0, w1, b1 ? 0x5410 : 0x7632), 4);
+  const uint32_t y0 = __byte_perm(w0, r, b1 ? 0x3254 : 0x5410), y1 = __byte_perm(w1, r, b1 ? 0x3276 : 0x7610);
+  r = __shfl_xor_sync(0xffffffffu, __byte_perm(y0, y1, b0 ? 0x6420 : 0x7531), 2);
+  w0 = __byte_perm(y0, r, b0 ? 0x3514 : 0x5240);
+  w1 = __byte_perm(y1, r, b0 ? 0x3716 : 0x7260);
+}
+
 // One launch runs the phases [f.phase_begin, f.phase_end): phase 0 = MLP1 (bias + SwiGLU -> e4m3 high/low
 // rows, args pa), phase 1 = MLP2 (bias -> fp16, args pb).  Run together, the pipeline state (stage ring,
-// accumulator buffers, scale slots) simply carries over from the last MLP1 item of a CTA to its first MLP2
-// item: no drain, no second prologue, and CTAs that are out of MLP1 items start on MLP2 while the others
+// accumulator buffers) simply carries over from the last MLP1 item of a CTA pair to its first MLP2
+// item: no drain, no second prologue, and pairs that are out of MLP1 items start on MLP2 while the others
 // finish.  An MLP2 item reads the SwiGLU rows of its token tile, which the MLP1 items of that tile (on any
-// SM) have written: every epilogue warp counts a finished MLP1 item into tile_done[tile] behind a fence, and
-// the producer waits (bounded) for the tile's count before it requests the tile's rows.  MLP1 items wait for
-// nothing and every CTA is resident (one per SM), so the MLP2 waits always end.
-__global__ void __launch_bounds__(kThreads, 1)
-expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__ CUtensorMap tm_x1,
-                   const __grid_constant__ CUtensorMap tm_w2, const __grid_constant__ CUtensorMap tm_x2,
-                   const GemmArgs pa, const GemmArgs pb, const MlpFuse f) {
+// SM) have written: kDoneWarp counts a finished MLP1 item of its CTA into tile_done[tile] behind a fence, and
+// the token producers wait (bounded) for the tile's count before they request the tile's rows; the weight
+// producers run ahead of that wait.  MLP1 items wait for nothing and every pair is resident (the grid is
+// what the device places at once), so the MLP2 waits always end.
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__ CUtensorMap tm_w1_last,
+                   const __grid_constant__ CUtensorMap tm_w2, const __grid_constant__ CUtensorMap tm_w2_last, const GemmArgs pa,
+                   const GemmArgs pb, const MlpFuse f) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t bar_base = smem_base + kBarOff;
   volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem_gen + kBarOff + 8 * kNumBars);
   uint32_t *tmem_slot = const_cast<uint32_t *>(abort_flag) + 1;
+  const uint32_t prog_base = smem_base + kProgOff;
 
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (kStages + s); };
   auto dfull_bar = [&](int d) { return bar_base + 8u * (2 * kStages + d); };
   auto dempty_bar = [&](int d) { return bar_base + 8u * (2 * kStages + 2 + d); };
-  auto sfa_full_bar = [&](int q) { return bar_base + 8u * (2 * kStages + 4 + q); };
-  auto sfa_empty_bar = [&](int q) { return bar_base + 8u * (2 * kStages + 4 + kSfaSlots + q); };
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(cluster_ctarank());   // 0 issues the MMAs of the pair
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+    // full: both producers; in the even CTA also the report that the odd CTA's half has landed
+    for (int s = 0; s < kStages; ++s) { mbar_init(full_bar(s), rank == 0 ? 3 : 2); mbar_init(empty_bar(s), 1); }
     for (int d = 0; d < 2; ++d) {
       mbar_init(dfull_bar(d), 1);
-      mbar_init(dempty_bar(d), kEpiWarps);
+      mbar_init(dempty_bar(d), 2 * kEpiWarps);   // the epilogue warps of both CTAs (even CTA's copy only)
     }
-    for (int q = 0; q < kSfaSlots; ++q) { mbar_init(sfa_full_bar(q), 1); mbar_init(sfa_empty_bar(q), 1); }
     *abort_flag = 0u;
+    for (int w = 0; w < kEpiWarps; ++w) st_release_cta(prog_base + 4u * w, 0u);
     fence_mbar_init();
     fence_proxy_async_smem();
   }
   if (warp == kMmaWarp) {
-    tmem_alloc(smem_u32(tmem_slot), kTmemCols);
-    tmem_relinquish();
+    tmem_alloc_pair(smem_u32(tmem_slot), kTmemCols);
+    tmem_relinquish_pair();
   }
-  if (warp == kProducerWarp && lane == 0) {
-    if (f.phase_begin == 0) { prefetch_tensormap(&tm_w1); prefetch_tensormap(&tm_x1); }
-    if (f.phase_end == 2) { prefetch_tensormap(&tm_w2); prefetch_tensormap(&tm_x2); }
+  if (warp == kWProducerWarp && lane == 0) {
+    if (f.phase_begin == 0) { prefetch_tensormap(&tm_w1); prefetch_tensormap(&tm_w1_last); }
+    if (f.phase_end == 2) { prefetch_tensormap(&tm_w2); prefetch_tensormap(&tm_w2_last); }
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync_all();   // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  // Items of a phase are dealt round-robin.  In a fused launch the MLP2 deal starts where the MLP1 deal
-  // ended, so that the CTAs with one MLP1 item more are not also the ones with one MLP2 item more.
+  // Items of a phase are dealt round-robin to the pairs.  In a fused launch the MLP2 deal starts where the MLP1
+  // deal ended, so that the pairs with one MLP1 item more are not also the ones with one MLP2 item more.
   const int n_work1 = *pa.n_work;
+  const int pairs = static_cast<int>(gridDim.x) >> 1, pair = static_cast<int>(blockIdx.x) >> 1;
   auto first_item = [&](int phase) -> int {
-    if (phase == 0 || f.phase_begin != 0) return static_cast<int>(blockIdx.x);
-    const int g = static_cast<int>(gridDim.x);
-    return (static_cast<int>(blockIdx.x) + g - n_work1 % g) % g;
+    if (phase == 0 || f.phase_begin != 0) return pair;
+    return (pair + pairs - n_work1 % pairs) % pairs;
   };
   unsigned int *status = pa.status;
+  bool ok = true;
 
-  if (warp == kProducerWarp) {
-    // ------------------------------------------------------------- TMA producer
-    // The warp stays converged; one elected lane issues the copies.
-    uint32_t item = 0, s = 0, e_par = 1u;   // a fresh stage passes the first wait
-    bool ok = true;
-    bool all_done = f.tile_done == nullptr;   // every MLP1 item of the launch is finished: no more checks
+  if (warp == kWProducerWarp) {
+    // ------------------------------------------------------------- weight producer
+    uint32_t s = 0, e_par = 1u;   // a fresh stage passes the first wait
     const uint64_t w_policy = l2_policy_evict_first();
    for (int phase = f.phase_begin; ok && phase < f.phase_end; ++phase) {
     const bool second = phase != 0;
-    const CUtensorMap *tm_w = second ? &tm_w2 : &tm_w1, *tm_x = second ? &tm_x2 : &tm_x1;
+    const CUtensorMap *tm_w = second ? &tm_w2 : &tm_w1, *tm_last = second ? &tm_w2_last : &tm_w1_last;
     const WorkItem *work = second ? pb.work : pa.work;
     const int n_work = second ? *pb.n_work : n_work1;
     const int nkc = second ? pb.n_kchunks : pa.n_kchunks, n_ntiles = second ? pb.n_ntiles : pa.n_ntiles;
-    const uint8_t *sfa = second ? pb.sfa : pa.sfa, *w_tiles = second ? pb.w_tiles : pa.w_tiles;
-    const int sfa_tile_stride = second ? pb.sfa_tile_stride : pa.sfa_tile_stride;
+    const uint8_t *w_tiles = second ? pb.w_tiles : pa.w_tiles;
     const int first = first_item(phase);
     WorkItem w_next = {};
     if (first < n_work) w_next = work[first];
-    for (int wi = first; ok && wi < n_work; wi += gridDim.x) {
+    for (int wi = first; ok && wi < n_work; wi += pairs) {
       const WorkItem w = w_next;
-      if (wi + static_cast<int>(gridDim.x) < n_work) w_next = work[wi + gridDim.x];
-      for (int blk = 0; ok && blk < w.nblk; ++blk, ++item) {
-        if (second && !all_done) {
-          // the SwiGLU rows of this token tile: all MLP1 items of the tile (one per weight block; the index
-          // kernel emits single-block items) must have been counted in by their 16 epilogue warps
-          const long long t0 = clock64();
-          for (uint32_t spin = 0;; ++spin) {
-            const uint32_t total = __shfl_sync(0xffffffffu, ld_acquire_gpu(f.tile_done + f.total_slot), 0);
-            if (total >= static_cast<uint32_t>(kEpiWarps) * static_cast<uint32_t>(n_work1)) { all_done = true; break; }
-            const uint32_t mine = __shfl_sync(0xffffffffu, ld_acquire_gpu(f.tile_done + w.tile), 0);
-            if (mine >= static_cast<uint32_t>(f.done_per_tile)) break;
-            if ((spin & 15u) == 15u) {
-              const bool late = __any_sync(0xffffffffu, clock64() - t0 > kWaitCycles);
-              if (late || __any_sync(0xffffffffu, *abort_flag != 0u)) {
-                if (late && lane == 0) { *abort_flag = 1u; atomicOr(status, ST_WAIT_AREADY); }
-                ok = false;
-                break;
-              }
-            }
-          }
-          if (!ok) break;
-          // written with ordinary stores on other SMs, read by the copy engine here
-          asm volatile("fence.proxy.async;" ::: "memory");
-        }
-        // activation scale atom of this token tile, through its own ring so that the producer never waits
-        // for an epilogue; a slot is free once the MMAs of the item that used it are done
-        const uint32_t q = item % kSfaSlots;
-        if (!mbar_wait_warp(sfa_empty_bar(q), ((item / kSfaSlots) & 1u) ^ 1u, abort_flag, status, ST_WAIT_EMPTY)) { ok = false; break; }
+      if (wi + pairs < n_work) w_next = work[wi + pairs];
+      const int half = (w.expert * n_ntiles + w.ntile) * 2 + rank;
+      const uint8_t *tiles = w_tiles + static_cast<size_t>(half) * nkc * kWTileBytes;
+      // weights pass through once per step: they must not push the activations and the results out of L2
+      for (int kc = 0; kc < nkc; kc += kSlices, tiles += 2 * kWTileBytes) {
+        if (!mbar_wait_warp(empty_bar(s), e_par, abort_flag, status, ST_WAIT_EMPTY)) { ok = false; break; }
+        const uint32_t stage = smem_base + s * kStageBytes;
         if (elect_one()) {
-          mbar_arrive_expect_tx(sfa_full_bar(q), kSfAtomBytes);
-          bulk_load(smem_base + kSfaOff + q * kSfAtomBytes, sfa + static_cast<size_t>(w.tile) * sfa_tile_stride,
-                    kSfAtomBytes, sfa_full_bar(q));
-        }
-        const uint32_t tile0 = (static_cast<uint32_t>(w.expert) * n_ntiles + w.ntile + blk) * nkc;
-        for (int kc = 0; kc < nkc; ++kc) {
-          if (!mbar_wait_warp(empty_bar(s), e_par, abort_flag, status, ST_WAIT_EMPTY)) { ok = false; break; }
-          const uint32_t stage = smem_base + s * kStageBytes;
-          if (elect_one()) {
-            mbar_arrive_expect_tx(full_bar(s), kABytes + kWLoadBytes + kSfbChunkBytes);
-            // the weight tile first: it has the longer way (HBM; the activations come from L2).  Weights pass
-            // through once per step: they must not push the activations and the results out of L2
-            tma_load_3d_hint(stage + kABytes, tm_w, 0, 0, static_cast<int>(tile0 + kc), full_bar(s), w_policy);
-            bulk_load_hint(stage + kABytes + kWBytes, w_tiles + static_cast<size_t>(tile0 + kc) * kWTileStride + kWTileCodes,
-                           kSfbChunkBytes, full_bar(s), w_policy);
-            tma_load_2d(stage, tm_x, 0, (w.tile * nkc + kc) * kTileM, full_bar(s));   // one contiguous 16 KB tile
+          if (kc + 1 < nkc) {
+            mbar_arrive_expect_tx(full_bar(s), 2 * (kWLoadBytes + kSfAtomBytes));
+            tma_load_5d_hint(stage, tm_w, 0, 0, 0, kc >> 1, half, full_bar(s), w_policy);
+            bulk_load_hint(stage + kSfaOff, tiles + 2 * kWTileCodes, 2 * kSfAtomBytes, full_bar(s), w_policy);
+          } else {
+            mbar_arrive_expect_tx(full_bar(s), kWLoadBytes + kSfAtomBytes);
+            tma_load_3d_hint(stage, tm_last, 0, 0, half, full_bar(s), w_policy);
+            bulk_load_hint(stage + kSfaOff, tiles + kWTileCodes, kSfAtomBytes, full_bar(s), w_policy);
           }
-          if (++s == kStages) { s = 0; e_par ^= 1u; }
         }
+        if (++s == kStages) { s = 0; e_par ^= 1u; }
       }
     }
    }
-    if (!ok) {  // give copies in flight time to land before the CTA's shared memory is released
-      for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+  } else if (warp == kXProducerWarp) {
+    // ------------------------------------------------------------- token producer
+    uint32_t s = 0, e_par = 1u;
+    bool all_done = f.tile_done == nullptr;   // every MLP1 item of the launch is finished: no more checks
+   for (int phase = f.phase_begin; ok && phase < f.phase_end; ++phase) {
+    const bool second = phase != 0;
+    const WorkItem *work = second ? pb.work : pa.work;
+    const int n_work = second ? *pb.n_work : n_work1;
+    const int nkc = second ? pb.n_kchunks : pa.n_kchunks;
+    const uint8_t *xq = second ? pb.xq : pa.xq, *sfb = second ? pb.sfb : pa.sfb;
+    const int sfb_tile_stride = second ? pb.sfb_tile_stride : pa.sfb_tile_stride;
+    const int first = first_item(phase);
+    WorkItem w_next = {};
+    if (first < n_work) w_next = work[first];
+    for (int wi = first; ok && wi < n_work; wi += pairs) {
+      const WorkItem w = w_next;
+      if (wi + pairs < n_work) w_next = work[wi + pairs];
+      if (second && !all_done) {
+        // the SwiGLU rows of this token tile: all MLP1 items of the tile (one per weight block) must have been
+        // counted in by both CTAs of their pair
+        const long long t0 = clock64();
+        for (uint32_t spin = 0;; ++spin) {
+          const uint32_t total = __shfl_sync(0xffffffffu, ld_acquire_gpu(f.tile_done + f.total_slot), 0);
+          if (total >= 2u * static_cast<uint32_t>(n_work1)) { all_done = true; break; }
+          const uint32_t mine = __shfl_sync(0xffffffffu, ld_acquire_gpu(f.tile_done + w.tile), 0);
+          if (mine >= static_cast<uint32_t>(f.done_per_tile)) break;
+          if ((spin & 15u) == 15u) {
+            const bool late = __any_sync(0xffffffffu, clock64() - t0 > kWaitCycles);
+            if (late || __any_sync(0xffffffffu, *abort_flag != 0u)) {
+              if (late && lane == 0) { *abort_flag = 1u; atomicOr(status, ST_WAIT_AREADY); }
+              ok = false;
+              break;
+            }
+          }
+        }
+        if (!ok) break;
+        // written with ordinary stores on other SMs, read by the copy engine here
+        asm volatile("fence.proxy.async;" ::: "memory");
+      }
+      // this CTA's half of the tile's rows (both slices of a pair; of a single last slice the unused other half too)
+      const uint32_t bytes = static_cast<uint32_t>(tile_n(w.ntok)) * kChunkK;
+      const uint8_t *src = xq + static_cast<size_t>(w.tile) * slice_pairs(nkc) * kPairBytes + rank * (kPairBytes / 2);
+      for (int kc = 0; kc < nkc; kc += kSlices, src += kPairBytes) {
+        if (!mbar_wait_warp(empty_bar(s), e_par, abort_flag, status, ST_WAIT_EMPTY)) { ok = false; break; }
+        const uint32_t stage = smem_base + s * kStageBytes;
+        if (elect_one()) {
+          mbar_arrive_expect_tx(full_bar(s), bytes + (kc == 0 ? kSfbTileBytes : 0));
+          if (kc == 0)
+            bulk_load(stage + kSfbOff, sfb + static_cast<size_t>(w.tile) * sfb_tile_stride, kSfbTileBytes, full_bar(s));
+          bulk_load(stage + kXOff, src, bytes, full_bar(s));
+        }
+        if (++s == kStages) { s = 0; e_par ^= 1u; }
+      }
     }
+   }
+  } else if (warp == kMmaWarp && rank != 0) {
+    // ------------------------------------------------------------- odd CTA: report landed slices to the even one
+    uint32_t s = 0, f_par = 0;
+   for (int phase = f.phase_begin; ok && phase < f.phase_end; ++phase) {
+    const bool second = phase != 0;
+    const int n_work = second ? *pb.n_work : n_work1;
+    const int nkc = second ? pb.n_kchunks : pa.n_kchunks;
+    for (int wi = first_item(phase); ok && wi < n_work; wi += pairs)
+      for (int kc = 0; kc < nkc; kc += kSlices) {
+        if (!mbar_wait_warp(full_bar(s), f_par, abort_flag, status, ST_WAIT_FULL)) { ok = false; break; }
+        if (elect_one()) mbar_arrive_cluster(full_bar(s), 0);
+        if (++s == kStages) { s = 0; f_par ^= 1u; }
+      }
+   }
   } else if (warp == kMmaWarp) {
-    // ------------------------------------------------------------- MMA issuer
+    // ------------------------------------------------------------- even CTA: MMA issuer of the pair
     // The warp stays converged and one elected lane issues the tcgen05 instructions, so that their operands
     // live in uniform registers.  The weights and activations need no tcgen05 fence after their wait (copy
     // engine and tensor core meet through the mbarrier); the accumulator hand-over from the epilogue does.
     const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
-    uint32_t item = 0, s = 0, f_par = 0, sfb_sel = 0;
-    bool ok = true;
-    const uint64_t desc_fixed = smem_desc_sw128(0);
+    uint32_t item = 0, s = 0, f_par = 0, sfa_sel = 0;
+    const uint64_t desc_w = smem_desc_sw128(0), desc_x = smem_desc_sw128(0, 2048);   // slices alternate in the token rows
    for (int phase = f.phase_begin; ok && phase < f.phase_end; ++phase) {
     const bool second = phase != 0;
     const WorkItem *work = second ? pb.work : pa.work;
@@ -238,213 +306,231 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
     const int K = second ? pb.K : pa.K, nkc = second ? pb.n_kchunks : pa.n_kchunks;
     const int full_chunks = K / kChunkK, tail_steps = (K % kChunkK) / 32;
     const int first = first_item(phase);
-    uint32_t nblk_next = 0;
-    if (first < n_work) nblk_next = work[first].nblk;
-    for (int wi = first; ok && wi < n_work; wi += gridDim.x) {
-      const uint32_t nblk = nblk_next;
-      if (wi + static_cast<int>(gridDim.x) < n_work) nblk_next = work[wi + gridDim.x].nblk;
-      for (uint32_t blk = 0; ok && blk < nblk; ++blk, ++item) {
-        const uint32_t d = item & 1u;
-        if (!mbar_wait_warp(dempty_bar(d), ((item >> 1) & 1u) ^ 1u, abort_flag, status, ST_WAIT_DEMPTY)) { ok = false; break; }
-        const uint32_t q = item % kSfaSlots;
-        if (!mbar_wait_warp(sfa_full_bar(q), (item / kSfaSlots) & 1u, abort_flag, status, ST_WAIT_AREADY)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t sfa_t = tm + kSfaCol0 + 4 * d;
-        if (elect_one()) tmem_cp_sf_atom(sfa_t, smem_base + kSfaOff + q * kSfAtomBytes);
-        const uint32_t d_addr = tm + d * kAccBufCols;
-        for (int kc = 0; kc < nkc; ++kc) {
-          if (!mbar_wait_warp(full_bar(s), f_par, abort_flag, status, ST_WAIT_FULL)) { ok = false; break; }
-          const uint32_t stage = smem_base + s * kStageBytes;
-          const uint32_t sfb_t = tm + kSfbCol0 + 8 * sfb_sel;
-          const uint64_t adesc = desc_fixed | (stage >> 4), bdesc = desc_fixed | ((stage + kABytes) >> 4);
-          if (elect_one()) {
-            tmem_cp_sf_atom(sfb_t, stage + kABytes + kWBytes);
-            tmem_cp_sf_atom(sfb_t + 4, stage + kABytes + kWBytes + kSfAtomBytes);
-            if (kc < full_chunks) {
-              mma_mxf8f6f4_ss(d_addr, adesc, bdesc, idesc_mxf8f6f4_m128(kTileN, 0), kc != 0, sfa_t, sfb_t);
-              mma_mxf8f6f4_ss(d_addr, adesc + 2, bdesc + 2, idesc_mxf8f6f4_m128(kTileN, 1), 1u, sfa_t, sfb_t);
-              mma_mxf8f6f4_ss(d_addr, adesc + 4, bdesc + 4, idesc_mxf8f6f4_m128(kTileN, 2), 1u, sfa_t, sfb_t);
-              mma_mxf8f6f4_ss(d_addr, adesc + 6, bdesc + 6, idesc_mxf8f6f4_m128(kTileN, 3), 1u, sfa_t, sfb_t);
-            } else {
-              for (int kb = 0; kb < tail_steps; ++kb)
-                mma_mxf8f6f4_ss(d_addr, adesc + 2 * kb, bdesc + 2 * kb, idesc_mxf8f6f4_m128(kTileN, kb), (kc | kb) != 0,
-                                sfa_t, sfb_t);
-            }
-            mma_commit(empty_bar(s));
-          }
-          if (++s == kStages) { s = 0; f_par ^= 1u; }
-          sfb_sel ^= 1u;
+    int ntok_next = 0;
+    if (first < n_work) ntok_next = work[first].ntok;
+    for (int wi = first; ok && wi < n_work; wi += pairs, ++item) {
+      const uint32_t n = __shfl_sync(0xffffffffu, static_cast<uint32_t>(tile_n(ntok_next)), 0);
+      if (wi + pairs < n_work) ntok_next = work[wi + pairs].ntok;
+      const uint32_t d = item & 1u;
+      if (!mbar_wait_warp(dempty_bar(d), ((item >> 1) & 1u) ^ 1u, abort_flag, status, ST_WAIT_DEMPTY)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t sfb_t = tm + kSfbCol0 + 8 * d;
+      const uint32_t d_addr = tm + d * kAccBufCols;
+      const uint32_t idesc = idesc_mxf8f6f4_m256(n, 0);
+      auto mma_slice = [&](uint32_t sl, uint32_t stage, int steps, bool first) {   // one elected lane
+        const uint32_t sfa_t = tm + kSfaCol0 + 4 * (sfa_sel + sl);
+        const uint64_t adesc = desc_w | ((stage + sl * kWBytes) >> 4);
+        const uint64_t bdesc = desc_x | ((stage + kXOff + sl * 1024) >> 4);
+        tmem_cp_sf_atom_pair(sfa_t, stage + kSfaOff + sl * kSfAtomBytes);
+        if (steps == 4) {
+          mma_mxf8f6f4_pair(d_addr, adesc, bdesc, idesc, first ? 0u : 1u, sfa_t, sfb_t);
+          mma_mxf8f6f4_pair(d_addr, adesc + 2, bdesc + 2, idesc | idesc_sf_id(1), 1u, sfa_t, sfb_t);
+          mma_mxf8f6f4_pair(d_addr, adesc + 4, bdesc + 4, idesc | idesc_sf_id(2), 1u, sfa_t, sfb_t);
+          mma_mxf8f6f4_pair(d_addr, adesc + 6, bdesc + 6, idesc | idesc_sf_id(3), 1u, sfa_t, sfb_t);
+        } else {
+          for (int kb = 0; kb < steps; ++kb)
+            mma_mxf8f6f4_pair(d_addr, adesc + 2 * kb, bdesc + 2 * kb, idesc | idesc_sf_id(kb), first && kb == 0 ? 0u : 1u, sfa_t, sfb_t);
         }
-        if (ok && elect_one()) {
-          mma_commit(dfull_bar(d));
-          mma_commit(sfa_empty_bar(q));
+      };
+      for (int kc = 0; kc < nkc; kc += kSlices) {
+        if (!mbar_wait_warp(full_bar(s), f_par, abort_flag, status, ST_WAIT_FULL)) { ok = false; break; }
+        const uint32_t stage = smem_base + s * kStageBytes;
+        if (elect_one()) {
+          if (kc == 0) {
+            tmem_cp_sf_atom_pair(sfb_t, stage + kSfbOff);
+            tmem_cp_sf_atom_pair(sfb_t + 4, stage + kSfbOff + kSfAtomBytes);
+          }
+          if (kc + kSlices <= full_chunks) {
+            mma_slice(0, stage, 4, kc == 0);
+            mma_slice(1, stage, 4, false);
+          } else {
+            for (int k = kc; k < min(nkc, kc + kSlices); ++k) mma_slice(k - kc, stage, k < full_chunks ? 4 : tail_steps, k == 0);
+          }
+          mma_commit_pair(empty_bar(s));
+        }
+        if (++s == kStages) { s = 0; f_par ^= 1u; }
+        sfa_sel ^= 2u;
+      }
+      if (ok && elect_one()) mma_commit_pair(dfull_bar(d));
+    }
+   }
+  } else if (warp == kDoneWarp) {
+    // ------------------------------------------------------------- counts finished MLP1 items
+    // A fence takes about as long as a small item: here it stays out of the epilogue warps' way, and one fence
+    // serves all items that every one of them has finished since the last.
+    if (f.phase_begin == 0 && f.tile_done != nullptr) {
+      uint32_t published = 0;
+      const uint32_t mine = pair < n_work1 ? static_cast<uint32_t>((n_work1 - 1 - pair) / pairs + 1) : 0u;
+      long long t0 = clock64();
+      for (uint32_t spin = 0; published < mine; ++spin) {
+        const uint32_t done = __reduce_min_sync(0xffffffffu, ld_acquire_cta(prog_base + 4u * (lane % kEpiWarps)));
+        if (done > published) {
+          __threadfence();
+          __syncwarp();
+          for (uint32_t i = published + lane; i < done; i += 32)
+            atomicAdd(f.tile_done + pa.work[pair + static_cast<int>(i) * pairs].tile, 1u);
+          if (lane == 0) atomicAdd(f.tile_done + f.total_slot, done - published);
+          published = done;
+          t0 = clock64();
+          spin = 0;
+        } else {
+          if ((spin & 63u) == 63u) {   // the MMA and copy roles record what went wrong; this one only leaves
+            if (__any_sync(0xffffffffu, *abort_flag != 0u || clock64() - t0 > 2 * kWaitCycles)) break;
+          }
+          __nanosleep(100);
         }
       }
     }
-   }
   } else {
     // ------------------------------------------------------------- epilogue warps
-    // Warp w reads tensor-memory lanes 32*(w%4).., i.e. accumulator rows 32q + l: token 16q + l/2, high
-    // (even l) or low (odd l) term.  Warps 4g..4g+3 take the 16-column chunks 4g..4g+3 (15 chunks in all).
-    // Loads are software pipelined: chunk c+1 is in flight while chunk c is processed.
-    const int quad = warp & 3, half = warp >> 2;
+    // Warp w reads tensor-memory lanes 32*(w%4)..: lane l of quadrant q is weight row 32q + l of this CTA's 120;
+    // neighbouring columns are the high and the low term of a token (x_operand_row).  Warps 4g..4g+3 take every
+    // fourth chunk of 16 columns; the next chunk's load is in flight while one is processed.
+    const int quad = warp & 3, grp = warp >> 2;
     const uint32_t lane_field = static_cast<uint32_t>(quad * 32) << 16;
     const int odd = lane & 1;
-    const int tok = quad * 16 + (lane >> 1);
+    const int lrow = quad * 32 + lane, q4 = (lane >> 1) & 3;
     const float h_scale = exp2f(static_cast<float>(-pa.h_exp));
     uint32_t item = 0;
-    bool ok = true;
    for (int phase = f.phase_begin; ok && phase < f.phase_end; ++phase) {
     const bool second = phase != 0;
     const WorkItem *work = second ? pb.work : pa.work;
     const int n_work = second ? *pb.n_work : n_work1;
     const int R = second ? pb.R : pa.R;
+    const bool add_bias = !second || pb.add_bias;
     const __nv_bfloat16 *bias = second ? pb.bias : pa.bias;
     const int first = first_item(phase);
     WorkItem w_next = {};
     if (first < n_work) w_next = work[first];
-    for (int wi = first; ok && wi < n_work; wi += gridDim.x) {
-     const WorkItem w = w_next;
-     if (wi + static_cast<int>(gridDim.x) < n_work) w_next = work[wi + gridDim.x];  // in flight during the wait below
-     for (int blk = 0; ok && blk < w.nblk; ++blk, ++item) {
+    for (int wi = first; ok && wi < n_work; wi += pairs, ++item) {
+      const WorkItem w = w_next;
+      if (wi + pairs < n_work) w_next = work[wi + pairs];  // in flight during the wait below
       const uint32_t d = item & 1u;
-      if (!mbar_wait(dfull_bar(d), (item >> 1) & 1u, abort_flag, status, ST_WAIT_DFULL)) { ok = false; break; }
+      const int n0 = w.ntile * kBlockRows + rank * kHalfRows;   // first weight row of this CTA's half
+      const bool row_ok = lrow < kHalfRows && n0 + lrow < R;
+      const float b = row_ok && add_bias ? __bfloat162float(bias[static_cast<size_t>(w.expert) * R + n0 + lrow]) : 0.f;
+      const int n_chunks = tile_n(w.ntok) / 16;   // 8 tokens each, and as many 4-token groups per CTA
+      if (!mbar_wait_warp(dfull_bar(d), (item >> 1) & 1u, abort_flag, status, ST_WAIT_DFULL)) { ok = false; break; }
       tc_fence_after();
-      const int n0 = (w.ntile + blk) * kTileN;
-      const bool tok_ok = tok < w.ntok;
-      const __nv_bfloat16 *bias_row = bias + static_cast<size_t>(w.expert) * R;
       const uint32_t acc = tmem_base + lane_field + d * kAccBufCols;
-      // chunks of this warp that hold rows of the matrix (rows past it are zero-filled and produce nothing)
-      const int c_beg = half * kEpiChunks;
-      const int c_end = min(min(c_beg + kEpiChunks, kTileN / 16), (R - n0 + 15) / 16);
-
-      auto process = [&](const uint32_t (&v)[16], int c0) {
-        // Sum of the high and low partial products of a token (adjacent lanes).  Each lane of the pair keeps 8
-        // of the 16 columns: the even lane columns 0-7, the odd lane 8-15 (MLP1: whole gate/up pairs, 4 outputs
-        // each; MLP2: 8 fp16 values, one 16-byte store, the pair's two stores fill one 32-byte sector).
-        float tot[8];
+      auto release = [&]() {   // the accumulator is in registers (or not this warp's business): the MMAs may go on
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(dempty_bar(d), 0);
+      };
+      auto process = [&](const uint32_t (&v)[16], int c) {
+        // Sum of the high and low partial products, plus the bias of this lane's row.  Of a pair of lanes (rows
+        // 2j, 2j+1) the even one finishes the first four tokens of the chunk, the odd one the others.
+        const int grp4 = 2 * c + odd;   // the lane's group of 8 columns; the even CTA's groups come first
+        const int t0 = (grp4 < n_chunks ? 2 * grp4 : 2 * (grp4 - n_chunks) + 1) * 4;
+        float even_row[4], odd_row[4];   // MLP1: gate, up; MLP2: two neighbouring outputs
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int ce = i, co = i + 8;   // columns the even / the odd lane keeps
-          const float fe = __uint_as_float(v[ce]), fo = __uint_as_float(v[co]);
-          const float mine = odd ? fo : fe;
-          const float give = odd ? fe : fo;
-          tot[i] = mine + __shfl_xor_sync(0xffffffffu, give, 1);
+        for (int i = 0; i < 4; ++i) {
+          const float lo = __uint_as_float(v[2 * i]) + __uint_as_float(v[2 * i + 1]) + b;
+          const float hi = __uint_as_float(v[2 * i + 8]) + __uint_as_float(v[2 * i + 9]) + b;
+          const float got = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1);
+          even_row[i] = odd ? got : lo;
+          odd_row[i] = odd ? hi : got;
         }
         if (!second) {
-          const int nc = n0 + c0 + 8 * odd;  // first of this lane's 8 columns
-          float b[8];
-          if (nc < R) {
-            const uint4 bv = __ldg(reinterpret_cast<const uint4 *>(bias_row + nc));
-            const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              b[2 * i] = __uint_as_float(bw[i] << 16);
-              b[2 * i + 1] = __uint_as_float(bw[i] & 0xffff0000u);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) b[i] = 0.f;
-          }
           float hs[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            hs[i] = swiglu_clamped(tot[2 * i] + b[2 * i], tot[2 * i + 1] + b[2 * i + 1], pa.limit, pa.alpha) * h_scale;
-          const uint32_t hi4 = pack_e4m3x4(hs[0], hs[1], hs[2], hs[3]);
-          float r[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) r[i] = (hs[i] - e4m3_to_float((hi4 >> (8 * i)) & 0xffu)) * 16.0f;
-          const uint32_t lo4 = pack_e4m3x4(r[0], r[1], r[2], r[3]);
-          const int j = pa.hq_joff + (nc >> 1);  // this lane's 4 intermediate features, as columns of MLP2's k window
-          if (tok_ok && nc < R) {
-            // MLP2's activation tiles: [tile][k slice][128 rows][128 bytes]
-            uint8_t *dst = pa.hq_out + ((static_cast<size_t>(w.tile) * pa.hq_nkc + (j >> 7)) * kTileM + 2 * tok) * kChunkK + (j & 127);
-            *reinterpret_cast<uint32_t *>(dst) = hi4;
-            *reinterpret_cast<uint32_t *>(dst + kChunkK) = lo4;
+          for (int i = 0; i < 4; ++i) hs[i] = swiglu_clamped(even_row[i], odd_row[i], pa.limit, pa.alpha) * h_scale;
+          const uint32_t h0 = pack_e4m3x2(hs[0], hs[1]), h1 = pack_e4m3x2(hs[2], hs[3]);
+          const float2 f0 = unpack_e4m3x2(h0), f1 = unpack_e4m3x2(h1);
+          const uint32_t l0 = pack_e4m3x2((hs[0] - f0.x) * 16.0f, (hs[1] - f0.y) * 16.0f);
+          const uint32_t l1 = pack_e4m3x2((hs[2] - f1.x) * 16.0f, (hs[3] - f1.y) * 16.0f);
+          uint32_t hi4 = h0 | (h1 << 16), lo4 = l0 | (l1 << 16);
+          transpose_pair(hi4, lo4, q4);   // four tokens of one feature per word -> four features of one token
+          const int grow = quad * 32 + (lane & 24);   // first weight row of the lane group: 4 intermediate features
+          if (grow < kHalfRows && n0 + grow < R && t0 + q4 < w.ntok) {
+            const int j = pa.hq_joff + (n0 + grow) / 2;   // their column in MLP2's k window
+            uint8_t *pr = pa.hq_out + (static_cast<size_t>(w.tile) * slice_pairs(pa.hq_nkc) + (j >> 8)) * kPairBytes;
+            *reinterpret_cast<uint32_t *>(pr + x_pair_offset(t0 + q4, 0, j & 255)) = hi4;
+            *reinterpret_cast<uint32_t *>(pr + x_pair_offset(t0 + q4, 1, j & 255)) = lo4;
           }
-        } else {
-          const int na = n0 + c0 + 8 * odd;  // first of this lane's 8 columns
-          if (tok_ok && na < R) {          // R is a multiple of 32 here, so the whole chunk is inside
-            float b[8];
-            if (pb.add_bias) {
-              const uint4 bv = __ldg(reinterpret_cast<const uint4 *>(bias_row + na));
-              const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+        } else if (row_ok) {   // R is a multiple of 32 here: both rows of a lane pair exist or neither does
+          // fp16 keeps 11 significant bits of a value that the combine will round to 8; what it cannot hold
+          // is a magnitude above 65504, which is reported, not stored silently as infinity
+          float big = 0.f;
+          __half *dst = pb.y_out + static_cast<size_t>(w.row0 + t0) * pb.ld_out + n0 + (lrow & ~1);
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                b[2 * i] = __uint_as_float(bw[i] << 16);
-                b[2 * i + 1] = __uint_as_float(bw[i] & 0xffff0000u);
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) b[i] = 0.f;
+          for (int i = 0; i < 4; ++i) {
+            if (t0 + i < w.ntok) {
+              big = fmaxf(big, fmaxf(fabsf(even_row[i]), fabsf(odd_row[i])));
+              *reinterpret_cast<__half2 *>(dst + static_cast<size_t>(i) * pb.ld_out) = __floats2half2_rn(even_row[i], odd_row[i]);
             }
-            // fp16 keeps 11 significant bits of a value that the combine will round to 8; what it cannot hold
-            // is a magnitude above 65504, which is reported, not stored silently as infinity
-            uint32_t o[4];
-            float big = 0.f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float y0 = tot[2 * i] + b[2 * i], y1 = tot[2 * i + 1] + b[2 * i + 1];
-              big = fmaxf(big, fmaxf(fabsf(y0), fabsf(y1)));
-              const __half2 hh = __floats2half2_rn(y0, y1);
-              o[i] = *reinterpret_cast<const uint32_t *>(&hh);
-            }
-            if (big > 65504.f) atomicOr(status, ST_Y_RANGE);
-            __half *dst = pb.y_out + static_cast<size_t>(w.row0 + tok) * pb.ld_out + na;
-            *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
           }
+          if (big > 65504.f) atomicOr(status, ST_Y_RANGE);
         }
       };
-
+      constexpr int kStep = kEpiWarps / 4;
       uint32_t va[16], vb[16];
-      int c = c_beg;
-      if (c < c_end) tmem_ld16(acc + c * 16, va);
-      while (c < c_end) {
+      if (grp < n_chunks) tmem_ld16(acc + grp * 16, va);
+      else release();
+      for (int c = grp; c < n_chunks; c += 2 * kStep) {
         tmem_wait_ld();
-        if (c + 1 < c_end) tmem_ld16(acc + (c + 1) * 16, vb);
-        process(va, c * 16);
-        if (++c >= c_end) break;
+        if (c + kStep < n_chunks) tmem_ld16(acc + (c + kStep) * 16, vb);
+        else release();
+        process(va, c);
+        if (c + kStep >= n_chunks) break;
         tmem_wait_ld();
-        if (c + 1 < c_end) tmem_ld16(acc + (c + 1) * 16, va);
-        process(vb, c * 16);
-        ++c;
+        if (c + 2 * kStep < n_chunks) tmem_ld16(acc + (c + 2 * kStep) * 16, va);
+        else release();
+        process(vb, c + kStep);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(dempty_bar(d));
-      if (!second && f.tile_done != nullptr) {
-        // this warp's SwiGLU rows of the item are written: fence by every lane, then one count per warp
-        __threadfence();
+      if (!second && f.tile_done != nullptr) {   // this warp's SwiGLU rows of the item are written
         __syncwarp();
-        if (lane == 0) {
-          atomicAdd(f.tile_done + w.tile, 1u);
-          atomicAdd(f.tile_done + f.total_slot, 1u);
-        }
+        if (lane == 0) st_release_cta(prog_base + 4u * warp, item + 1u);
       }
-     }
     }
    }
   }
 
+  if (!ok && warp >= kWProducerWarp) {  // give copies in flight time to land before shared memory is released
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+  }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
+  cluster_sync_all();   // neither CTA leaves while the pair's MMAs or reports may still touch its memory
   if (warp == kMmaWarp) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTmemCols);
+    tmem_dealloc_pair(tmem_base, kTmemCols);
   }
 }
 
-cudaError_t expert_gemm_init() {
-  return cudaFuncSetAttribute(expert_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+// Per-device attributes; *grid receives the CTAs (two per pair) the device keeps resident at once, which the
+// waits of MLP2 items on MLP1 items rely on.
+cudaError_t expert_gemm_init(int *grid) {
+  cudaError_t e = cudaFuncSetAttribute(expert_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2, 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = kSmemBytes;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int pairs = 0;
+  e = cudaOccupancyMaxActiveClusters(&pairs, expert_gemm_kernel, &cfg);
+  if (e != cudaSuccess) return e;
+  if (pairs < 1) return cudaErrorLaunchOutOfResources;
+  *grid = 2 * pairs;
+  return cudaSuccess;
 }
 
 // Phases [f.phase_begin, f.phase_end) of the expert MLP in one launch: both in the usual call, one at a
 // time (two launches, f.tile_done = nullptr) on request.
-void launch_expert_mlp(const CUtensorMap &tm_w1, const CUtensorMap &tm_x1, const GemmArgs &a, const CUtensorMap &tm_w2,
-                       const CUtensorMap &tm_x2, const GemmArgs &b, const MlpFuse &f, int grid, cudaStream_t s) {
-  expert_gemm_kernel<<<grid, kThreads, kSmemBytes, s>>>(tm_w1, tm_x1, tm_w2, tm_x2, a, b, f);
+void launch_expert_mlp(const CUtensorMap (&tm_w1)[2], const GemmArgs &a, const CUtensorMap (&tm_w2)[2], const GemmArgs &b,
+                       const MlpFuse &f, int grid, cudaStream_t s) {
+  expert_gemm_kernel<<<grid, kThreads, kSmemBytes, s>>>(tm_w1[0], tm_w1[1], tm_w2[0], tm_w2[1], a, b, f);
 }
 
-int expert_mlp_done_per_tile(int n_ntiles1) { return kEpiWarps * n_ntiles1; }
+int expert_mlp_done_per_tile(int n_ntiles1) { return 2 * n_ntiles1; }
 
 }  // namespace moe

@@ -37,39 +37,30 @@ int fail(moe_ctx *c, int code, const char *fmt, ...) {
                   "%s failed: %s (%s:%d)", #expr, cudaGetErrorString(e__), __FILE__, __LINE__); \
   } while (0)
 
-// Weight tiles (LayerWeights::w1_tiles): every 16 KB tile starts with 240 rows x 64 bytes of packed e2m1 codes,
-// declared to TMA as 4-bit elements that it expands to the 8-bit containers of the block-scaled MMA
-// (16U4_ALIGN16B): dims {128 codes, 240 rows, tiles}, one box = the codes of one tile, a contiguous 15 KB read.
-int make_weight_map(moe_ctx *c, CUtensorMap *m, const uint8_t *base, size_t n_tiles) {
+// Tensor maps of the weight codes (LayerWeights::w1_tiles), declared to TMA as 4-bit elements that it expands to the
+// 8-bit containers of the block-scaled MMA (16U4_ALIGN16B).  m[0]: one box = the codes of a pair of k slices, a
+// contiguous 15 KB read; m[1]: the codes of the single last slice of an odd number.  A map of slices that do not
+// exist is made with one of them and never used.
+int make_weight_maps(moe_ctx *c, CUtensorMap (&m)[2], const uint8_t *base, size_t n_halves, int n_kc) {
   TensorMapEncodeFn fn = tensor_map_encoder();
   if (!fn) return fail(c, MOE_ERR_CUDA, "cuTensorMapEncodeTiled not available");
-  const cuuint64_t dims[3] = {kChunkK, kTileN, static_cast<cuuint64_t>(n_tiles)};
-  const cuuint64_t strides[2] = {kChunkK / 2, kWTileStride};
-  const cuuint32_t box[3] = {kChunkK, kTileN, 1};
-  const cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3, const_cast<uint8_t *>(base), dims, strides, box, es,
+  const cuuint64_t half = static_cast<cuuint64_t>(n_kc) * kWTileBytes;
+  const cuuint32_t es[5] = {1, 1, 1, 1, 1};
+  const cuuint64_t dims0[5] = {kChunkK, kHalfRows, 2, static_cast<cuuint64_t>(std::max(1, n_kc / 2)), n_halves};
+  const cuuint64_t strides0[4] = {kChunkK / 2, kWTileCodes, 2 * kWTileBytes, half};
+  const cuuint32_t box0[5] = {kChunkK, kHalfRows, 2, 1, 1};
+  CUresult r = fn(&m[0], CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 5, const_cast<uint8_t *>(base), dims0, strides0, box0, es,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(c, MOE_ERR_CUDA, "cuTensorMapEncodeTiled(weights, %zu tiles) -> %d", n_tiles, (int)r);
-  return MOE_OK;
-}
-
-// e4m3 activation tiles: [token tile][k slice][128 rows][128 bytes], so that the 16 KB a work item needs for one
-// k slice are one contiguous run (rows of K bytes would make the box 128 separate 128-byte pieces).  To TMA
-// this is a matrix of 128-byte rows; box = 128 x 128, 128-byte swizzle.
-int make_act_map(moe_ctx *c, CUtensorMap *m, const uint8_t *base, size_t n_tiles, int n_kc) {
-  TensorMapEncodeFn fn = tensor_map_encoder();
-  if (!fn) return fail(c, MOE_ERR_CUDA, "cuTensorMapEncodeTiled not available");
-  const cuuint64_t rows = static_cast<cuuint64_t>(n_tiles) * n_kc * kTileM;
-  const cuuint64_t dims[2] = {kChunkK, rows};
-  const cuuint64_t strides[1] = {kChunkK};
-  const cuuint32_t box[2] = {kChunkK, kTileM};
-  const cuuint32_t es[2] = {1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(base), dims, strides, box, es,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS)
-    return fail(c, MOE_ERR_CUDA, "cuTensorMapEncodeTiled(activations, %zu tiles x %d slices) -> %d", n_tiles, n_kc, (int)r);
+  if (r == CUDA_SUCCESS) {
+    const cuuint64_t dims1[3] = {kChunkK, kHalfRows, n_halves};
+    const cuuint64_t strides1[2] = {kChunkK / 2, half};
+    const cuuint32_t box1[3] = {kChunkK, kHalfRows, 1};
+    r = fn(&m[1], CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3, const_cast<uint8_t *>(base) + w_codes_offset((n_kc - 1) & ~1),
+           dims1, strides1, box1, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  }
+  if (r != CUDA_SUCCESS) return fail(c, MOE_ERR_CUDA, "cuTensorMapEncodeTiled(weights, %zu x %d slices) -> %d", n_halves, n_kc, (int)r);
   return MOE_OK;
 }
 
@@ -92,32 +83,29 @@ int dev_alloc(moe_ctx *c, T **p, size_t n) {
   return MOE_OK;
 }
 
-// One weight matrix -> the 16 KB tiles the GEMM streams (LayerWeights::w1_tiles).  codes: [E][R] rows of
-// row_bytes packed bytes at `pitch`; raw: E8M0 scales [E][R][nblk].  In a tile the scale of row r (of the tile's
-// 240), k block kb sits at byte (r%32)*16 + (r/32 %4)*4 + kb of atom r/128, the order tcgen05.cp puts them into
+// One weight matrix -> the tiles the GEMM streams (LayerWeights::w1_tiles).  codes: [E][R] rows of
+// row_bytes packed bytes at `pitch`; raw: E8M0 scales [E][R][nblk].  The scale of row r (of the tile's
+// 120), k block kb sits at byte (r%32)*16 + (r/32)*4 + kb of the atom, the order tcgen05.cp puts them into
 // tensor memory; 127 (scale 1) and zero codes where no row or no block exists.
 void tile_weights(const uint8_t *codes, size_t pitch, size_t row_bytes, const uint8_t *raw, int E, int R, int nblk,
                   int n_ntiles, int n_kc, std::vector<uint8_t> &out) {
-  out.assign(static_cast<size_t>(E) * n_ntiles * n_kc * kWTileStride, 0);
-  for (size_t t = 0; t < static_cast<size_t>(E) * n_ntiles * n_kc; ++t)
-    memset(&out[t * kWTileStride + kWTileCodes], 127, kSfbChunkBytes);
+  const size_t n_halves = static_cast<size_t>(E) * n_ntiles * 2, half_bytes = static_cast<size_t>(n_kc) * kWTileBytes;
+  out.assign(n_halves * half_bytes, 0);
+  for (size_t h = 0; h < n_halves; ++h)
+    for (int kc = 0; kc < n_kc; ++kc) memset(&out[h * half_bytes + w_scales_offset(kc, n_kc)], 127, kSfAtomBytes);
   for (int e = 0; e < E; ++e)
     for (int r = 0; r < R; ++r) {
       const uint8_t *src_c = codes + (static_cast<size_t>(e) * R + r) * pitch;
       const uint8_t *src_s = raw + (static_cast<size_t>(e) * R + r) * nblk;
-      const int nt = r / kTileN, rr = r % kTileN, atom = rr / 128, ra = rr % 128;
-      uint8_t *tile0 = &out[(static_cast<size_t>(e) * n_ntiles + nt) * n_kc * kWTileStride];
+      const int rr = r % kHalfRows;
+      uint8_t *half = &out[(static_cast<size_t>(e) * n_ntiles * 2 + r / kHalfRows) * half_bytes];
       for (int kc = 0; kc < n_kc; ++kc) {
         const size_t off = static_cast<size_t>(kc) * (kChunkK / 2);
         if (off < row_bytes)
-          memcpy(tile0 + static_cast<size_t>(kc) * kWTileStride + rr * (kChunkK / 2), src_c + off,
-                 std::min<size_t>(kChunkK / 2, row_bytes - off));
+          memcpy(half + w_codes_offset(kc) + rr * (kChunkK / 2), src_c + off, std::min<size_t>(kChunkK / 2, row_bytes - off));
       }
-      for (int b = 0; b < nblk; ++b) {
-        const int kc = b / 4, kb = b % 4;
-        tile0[static_cast<size_t>(kc) * kWTileStride + kWTileCodes + atom * kSfAtomBytes + (ra % 32) * 16 + (ra / 32) * 4 + kb] =
-            src_s[b];
-      }
+      for (int b = 0; b < nblk; ++b)
+        half[w_scales_offset(b / 4, n_kc) + (rr % 32) * 16 + (rr / 32) * 4 + b % 4] = src_s[b];
     }
 }
 
@@ -146,7 +134,7 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
   const bool tpcall = tp_rows_local > 0;
   const int tp = c->cfg.tp_size, rank = c->cfg.tp_rank;
   const int T = rows, P = rows * c->K, E = c->E, H = c->H, K = c->K;
-  const int n_nt1 = (c->R1 + kTileN - 1) / kTileN, n_nt2 = (H + kTileN - 1) / kTileN;
+  const int n_nt1 = (c->R1 + kBlockRows - 1) / kBlockRows, n_nt2 = (H + kBlockRows - 1) / kBlockRows;
 
   CU_TRY(c, cudaMemsetAsync(c->counts, 0, sizeof(int) * E, s));
   auto mark = [&]() {
@@ -237,7 +225,7 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
   }
   mark();
   if (flags & MOE_FWD_SIMT_GEMM) launch_gather_rows(t, c->row_token, c->offsets, E, c->xperm, H, P, s);
-  else launch_quantize_rows(t, c->pair_slot, T, K, c->xq, c->sfa_x, H, s);
+  else launch_quantize_rows(t, c->pair_slot, T, K, c->xq, c->sfb_x, H, s);
   mark();
   const int add_b2 = c->cfg.tp_rank == 0 ? 1 : 0;
   bool mlp_in_one_launch = false;
@@ -251,27 +239,27 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
     GemmArgs a{};
     a.work = c->work1; a.n_work = c->n_work; a.K = H; a.R = c->R1;
     a.n_kchunks = (H + kChunkK - 1) / kChunkK; a.n_ntiles = n_nt1;
-    a.w_tiles = w.w1_tiles; a.sfa = c->sfa_x; a.sfa_tile_stride = kSfAtomBytes; a.bias = w.b1; a.add_bias = 1;
+    a.w_tiles = w.w1_tiles; a.xq = c->xq; a.sfb = c->sfb_x; a.sfb_tile_stride = kSfbTileBytes; a.bias = w.b1; a.add_bias = 1;
     a.hq_out = c->hq; a.hq_joff = c->joff; a.hq_nkc = (c->Kw + kChunkK - 1) / kChunkK; a.y_out = nullptr; a.ld_out = c->Kw;
     a.h_exp = c->h_exp;
     a.limit = c->cfg.swiglu_limit; a.alpha = c->cfg.swiglu_alpha; a.status = status;
     GemmArgs b = a;
     b.work = c->work2; b.n_work = c->n_work + 1; b.K = c->Kw; b.R = H;
     b.n_kchunks = (c->Kw + kChunkK - 1) / kChunkK; b.n_ntiles = n_nt2;
-    b.w_tiles = w.w2_tiles; b.sfa = c->sfa_h; b.sfa_tile_stride = 0; b.bias = w.b2; b.add_bias = add_b2;
+    b.w_tiles = w.w2_tiles; b.xq = c->hq; b.sfb = c->sfb_h; b.sfb_tile_stride = 0; b.bias = w.b2; b.add_bias = add_b2;
     b.hq_out = nullptr; b.y_out = c->ybuf; b.ld_out = H;
     MlpFuse fuse{};
     fuse.total_slot = c->max_tiles;
     fuse.done_per_tile = expert_mlp_done_per_tile(n_nt1);
     if (flags & MOE_FWD_SPLIT_MLP) {   // MLP1 and MLP2 as two launches
       fuse.phase_begin = 0; fuse.phase_end = 1; fuse.tile_done = nullptr;
-      launch_expert_mlp(w.tm_w1, c->tm_x1, a, w.tm_w2, c->tm_x2, b, fuse, c->sm_count, s);
+      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, fuse, c->gemm_grid, s);
       mark();
       fuse.phase_begin = 1; fuse.phase_end = 2;
-      launch_expert_mlp(w.tm_w1, c->tm_x1, a, w.tm_w2, c->tm_x2, b, fuse, c->sm_count, s);
+      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, fuse, c->gemm_grid, s);
     } else {                           // one launch; the MLP2 stage of a profile is then empty
       fuse.phase_begin = 0; fuse.phase_end = 2; fuse.tile_done = c->tile_done;
-      launch_expert_mlp(w.tm_w1, c->tm_x1, a, w.tm_w2, c->tm_x2, b, fuse, c->sm_count, s);
+      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, fuse, c->gemm_grid, s);
       mark();
       c->launches -= 1;
       mlp_in_one_launch = true;
@@ -372,7 +360,7 @@ int moe_create(const moe_config *cfg, moe_handle *out) {
   if (prop.major != 10) return fail(c, MOE_ERR_NO_SM100, "device %d is sm_%d%d; this library is sm_100a only", cfg->device, prop.major, prop.minor);
   c->sm_count = prop.multiProcessorCount;
   CU_TRY(c, cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-  CU_TRY(c, expert_gemm_init());
+  CU_TRY(c, expert_gemm_init(&c->gemm_grid));
   CU_TRY(c, router_init(&c->router_cluster));
 
   const size_t T = c->max_rows, P = c->max_pairs;
@@ -409,8 +397,8 @@ int moe_create(const moe_config *cfg, moe_handle *out) {
   CU_TRY(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
   CU_TRY(c, cudaEventCreateWithFlags(&c->ev_fork2, cudaEventDisableTiming));
   CU_TRY(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
-  const int n_nt1 = (c->R1 + kTileN - 1) / kTileN, n_nt2 = (c->H + kTileN - 1) / kTileN;
-  c->max_tiles = c->max_pairs / kTokTile + c->E + 1;
+  const int n_nt1 = (c->R1 + kBlockRows - 1) / kBlockRows, n_nt2 = (c->H + kBlockRows - 1) / kBlockRows;
+  c->max_tiles = c->max_pairs / kMaxTileTok + c->E + 1;
   if ((rc = dev_alloc(c, &c->tile_done, static_cast<size_t>(c->max_tiles) + 1))) return rc;
   c->max_work1 = c->max_tiles * n_nt1;
   c->max_work2 = c->max_tiles * n_nt2;
@@ -421,23 +409,22 @@ int moe_create(const moe_config *cfg, moe_handle *out) {
     c->h_exp = static_cast<int>(ceilf(log2f(bound))) - 8;
   }
   const int n_kc1 = (c->H + kChunkK - 1) / kChunkK, n_kc2 = (c->Kw + kChunkK - 1) / kChunkK;
-  const size_t act_tile = static_cast<size_t>(kTileM) * kChunkK;   // 16 KB per (token tile, k slice)
-  const size_t xq_bytes = static_cast<size_t>(c->max_tiles) * n_kc1 * act_tile;
-  const size_t hq_bytes = static_cast<size_t>(c->max_tiles) * n_kc2 * act_tile;
+  const size_t xq_bytes = static_cast<size_t>(c->max_tiles) * slice_pairs(n_kc1) * kPairBytes;
+  const size_t hq_bytes = static_cast<size_t>(c->max_tiles) * slice_pairs(n_kc2) * kPairBytes;
   if ((rc = dev_alloc(c, &c->xq, xq_bytes))) return rc;
   if ((rc = dev_alloc(c, &c->hq, hq_bytes))) return rc;
-  if ((rc = dev_alloc(c, &c->sfa_x, static_cast<size_t>(c->max_tiles) * kSfAtomBytes))) return rc;
-  if ((rc = dev_alloc(c, &c->sfa_h, static_cast<size_t>(kSfAtomBytes)))) return rc;
+  if ((rc = dev_alloc(c, &c->sfb_x, static_cast<size_t>(c->max_tiles) * kSfbTileBytes))) return rc;
+  if ((rc = dev_alloc(c, &c->sfb_h, static_cast<size_t>(kSfbTileBytes)))) return rc;
   if ((rc = dev_alloc(c, &c->tile_base, static_cast<size_t>(c->E) + 1))) return rc;
   CU_TRY(c, cudaMemset(c->xq, 0, xq_bytes));   // bytes past K in the last slice and never-written columns stay 0
   CU_TRY(c, cudaMemset(c->hq, 0, hq_bytes));
-  CU_TRY(c, cudaMemset(c->sfa_x, 127, static_cast<size_t>(c->max_tiles) * kSfAtomBytes));
+  CU_TRY(c, cudaMemset(c->sfb_x, 127, static_cast<size_t>(c->max_tiles) * kSfbTileBytes));
   {
-    uint8_t atom[kSfAtomBytes];
-    for (int r = 0; r < kTileM; ++r)
+    uint8_t atoms[kSfbTileBytes];
+    for (int r = 0; r < 256; ++r)
       for (int kb = 0; kb < 4; ++kb)
-        atom[(r % 32) * 16 + (r / 32) * 4 + kb] = static_cast<uint8_t>(127 + c->h_exp - ((r & 1) ? 4 : 0));
-    CU_TRY(c, cudaMemcpy(c->sfa_h, atom, kSfAtomBytes, cudaMemcpyHostToDevice));
+        atoms[r / 128 * kSfAtomBytes + (r % 32) * 16 + (r / 32 % 4) * 4 + kb] = static_cast<uint8_t>(127 + c->h_exp - ((r & 1) ? 4 : 0));
+    CU_TRY(c, cudaMemcpy(c->sfb_h, atoms, kSfbTileBytes, cudaMemcpyHostToDevice));
   }
   if ((rc = dev_alloc(c, &c->work1, (size_t)c->max_work1))) return rc;
   if ((rc = dev_alloc(c, &c->work2, (size_t)c->max_work2))) return rc;
@@ -448,8 +435,6 @@ int moe_create(const moe_config *cfg, moe_handle *out) {
   // Rows past the current batch are read (and discarded) by token tiles that overhang; keep them finite.
   CU_TRY(c, cudaMemset(c->xperm, 0, P * c->H * sizeof(__half)));
   CU_TRY(c, cudaMemset(c->hbuf, 0, P * c->Kw * sizeof(__half)));
-  if ((rc = make_act_map(c, &c->tm_x1, c->xq, c->max_tiles, n_kc1))) return rc;
-  if ((rc = make_act_map(c, &c->tm_x2, c->hq, c->max_tiles, n_kc2))) return rc;
   return MOE_OK;
 }
 
@@ -478,7 +463,7 @@ int moe_destroy(moe_handle c) {
   cudaFree(c->offsets); cudaFree(c->pair_row); cudaFree(c->row_token); cudaFree(c->pair_slot); cudaFree(c->tile_done); cudaFree(c->xperm); cudaFree(c->hbuf);
   cudaFree(c->ybuf); cudaFree(c->out_f32); cudaFree(c->out_bf16); cudaFree(c->work1); cudaFree(c->work2);
   cudaFree(c->n_work); cudaFree(c->status);
-  cudaFree(c->xq); cudaFree(c->hq); cudaFree(c->sfa_x); cudaFree(c->sfa_h); cudaFree(c->tile_base);
+  cudaFree(c->xq); cudaFree(c->hq); cudaFree(c->sfb_x); cudaFree(c->sfb_h); cudaFree(c->tile_base);
   delete c;
   return MOE_OK;
 }
@@ -518,8 +503,8 @@ int moe_load_layer(moe_handle c, int layer, const uint8_t *w1_codes, const uint8
     for (uint8_t b : *sv)
       if (b == 0xFF) return fail(c, MOE_ERR_SCALE_RANGE, "layer %d: E8M0 scale byte 0xFF (NaN)", layer);
 
-  const int n_nt1 = (R1 + kTileN - 1) / kTileN, n_kc1 = (H + kChunkK - 1) / kChunkK;
-  const int n_nt2 = (H + kTileN - 1) / kTileN, n_kc2 = (Kw + kChunkK - 1) / kChunkK;
+  const int n_nt1 = (R1 + kBlockRows - 1) / kBlockRows, n_kc1 = (H + kChunkK - 1) / kChunkK;
+  const int n_nt2 = (H + kBlockRows - 1) / kBlockRows, n_kc2 = (Kw + kChunkK - 1) / kChunkK;
   std::vector<uint8_t> t1, t2;
   tile_weights(c1.data(), p1, w1_row, s1.data(), E, R1, H / 32, n_nt1, n_kc1, t1);
   tile_weights(c2.data(), p2, w2_row, s2.data(), E, H, Kw / 32, n_nt2, n_kc2, t2);
@@ -557,8 +542,8 @@ int moe_load_layer(moe_handle c, int layer, const uint8_t *w1_codes, const uint8
   CU_TRY(c, cudaMemcpy(w.b2, b2, static_cast<size_t>(E) * H * 2, cudaMemcpyHostToDevice));
   CU_TRY(c, cudaMemcpy(w.router_w3, w3.data(), w3.size() * 2, cudaMemcpyHostToDevice));
   CU_TRY(c, cudaMemcpy(w.router_b, router_b, static_cast<size_t>(E) * 4, cudaMemcpyHostToDevice));
-  if ((rc = make_weight_map(c, &w.tm_w1, w.w1_tiles, static_cast<size_t>(E) * n_nt1 * n_kc1))) return rc;
-  if ((rc = make_weight_map(c, &w.tm_w2, w.w2_tiles, static_cast<size_t>(E) * n_nt2 * n_kc2))) return rc;
+  if ((rc = make_weight_maps(c, w.tm_w1, w.w1_tiles, static_cast<size_t>(E) * n_nt1 * 2, n_kc1))) return rc;
+  if ((rc = make_weight_maps(c, w.tm_w2, w.w2_tiles, static_cast<size_t>(E) * n_nt2 * 2, n_kc2))) return rc;
   if (!make_router_weight_map(&w.tm_router, w.router_w3, E, H))
     return fail(c, MOE_ERR_CUDA, "cuTensorMapEncodeTiled(router weight, %d x %d) failed", E, H);
   w.loaded = true;

@@ -16,16 +16,53 @@
 namespace moe {
 
 // ---- tiling constants of the expert GEMM (expert_gemm_sm100.cu) -------------
-constexpr int kTileN = 240;        // weight rows per work item (UMMA N); divides 5760 and 2880
-constexpr int kTileNPad = 256;     // rows reserved per weight tile in shared memory / scale atoms
-constexpr int kChunkK = 128;       // reduction elements per shared-memory stage (4 MMA k-steps of 32)
-constexpr int kTokTile = 64;       // token rows per work item
-constexpr int kTileM = 2 * kTokTile;  // UMMA M: each token contributes a high and a low e4m3 row
+constexpr int kBlockRows = 240;    // weight rows per work item; divides 5760 and 2880
+constexpr int kHalfRows = kBlockRows / 2;  // weight rows per CTA of a pair: a weight tile
+constexpr int kChunkK = 128;       // reduction elements per slice (4 MMA k-steps of 32)
+constexpr int kMaxTileTok = 96;    // tokens per token tile, at most
+constexpr int kTileRows = 2 * kMaxTileTok;  // each token contributes a high and a low e4m3 row
+constexpr int kPairBytes = kTileRows * 2 * kChunkK;  // two k slices of a token tile: 49152 bytes
 constexpr int kSfAtomBytes = 512;  // scale factors of 128 rows x 4 k-blocks, tensor-memory order
-constexpr int kSfbChunkBytes = 2 * kSfAtomBytes;  // weight scales of one tile (240 rows in two atoms)
-constexpr int kWTileCodes = kTileN * kChunkK / 2;  // 15360 bytes of packed codes per weight tile
-constexpr int kWTileStride = kWTileCodes + kSfbChunkBytes;  // 16384: codes, then scales
-static_assert(kWTileStride == 16384, "weight tiles are 16 KB");
+constexpr int kSfbTileBytes = 2 * kSfAtomBytes;   // token scales of one tile (192 rows in two atoms)
+constexpr int kWTileCodes = kHalfRows * kChunkK / 2;  // 7680 bytes of packed codes per weight tile
+constexpr int kWTileBytes = kWTileCodes + kSfAtomBytes;  // 8192: codes and scales
+static_assert(kMaxTileTok % 8 == 0, "token tiles are cut in steps of 8 tokens");
+
+// Tokens per tile of an expert with cnt rows: as few tiles as hold them, of equal size in steps of 8 tokens (the
+// instruction's N moves in steps of 16 rows), so that no tile is a small rest.  No tile is empty: one less would
+// hold at most kMaxTileTok * (tiles - 1) < cnt rows.
+__host__ __device__ inline int expert_tiles(int cnt) { return (cnt + kMaxTileTok - 1) / kMaxTileTok; }
+__host__ __device__ inline int tokens_per_tile(int cnt) {
+  const int n = expert_tiles(cnt);
+  return n == 0 ? kMaxTileTok : ((cnt + n - 1) / n + 7) / 8 * 8;
+}
+__host__ __device__ inline int slice_pairs(int n_slices) { return (n_slices + 1) / 2; }
+
+// Token rows of a tile: [pair of k slices][CTA][8-row group][slice of the pair][8 rows][128 bytes].  Four tokens make
+// a group of 8 rows (high and low term each); even groups belong to the even CTA of the pair that works on the tile,
+// odd ones to the odd CTA, so that what one CTA needs of both slices is one contiguous run whatever the number of
+// tokens.  The eight 16-byte pieces of a row are permuted by the row (the 128-byte swizzle the tensor core reads).
+// Byte of (token, low term?, element) inside a tile's pair of slices; k is the element's position in the pair.
+__host__ __device__ inline int x_pair_offset(int tok, int low, int k) {
+  const int row = (tok & 3) * 2 + low;
+  return ((tok >> 2) & 1) * (kPairBytes / 2) + (tok >> 3) * 2048 + (k >> 7) * 1024 + row * kChunkK +
+         ((((k >> 4) ^ row) & 7) << 4) + (k & 15);
+}
+// Row of the instruction's N operand that holds the token's high term (the low term follows) in a tile with N = n:
+// the even CTA's groups come first.  The accumulator column and the scale row have the same number.
+__host__ __device__ inline int x_operand_row(int tok, int n) { return ((tok >> 2) & 1) * (n / 2) + (tok >> 3) * 8 + (tok & 3) * 2; }
+// Instruction N for a tile of ntok tokens: two rows per token, in the steps of 16 that M = 256 allows.
+__host__ __device__ inline int tile_n(int ntok) { return (2 * ntok + 15) & ~15; }
+
+// Weight tiles of one 120-row half of a block: pairs of k slices of 16 KB, [codes, 2 x 7680][scale atoms, 2 x 512],
+// then a single slice of 8 KB, [codes][scale atom], where their number is odd.  Byte of slice kc's codes and scales:
+__host__ __device__ inline size_t w_codes_offset(int kc) {
+  return static_cast<size_t>(kc >> 1) * 2 * kWTileBytes + (kc & 1) * kWTileCodes;
+}
+__host__ __device__ inline size_t w_scales_offset(int kc, int n_kc) {
+  const int in_pair = (kc | 1) < n_kc ? 2 : 1;   // slices stored together with this one
+  return static_cast<size_t>(kc >> 1) * 2 * kWTileBytes + in_pair * kWTileCodes + (kc & 1) * kSfAtomBytes;
+}
 
 // Device status bits (MOE_DBG_STATUS).
 enum : unsigned {
@@ -71,16 +108,14 @@ struct HostSlot {
   long long ticket = -1;                         // call that owns the slot; -1: free
 };
 
-// One work item of the grouped GEMM: one token tile against nblk adjacent kTileN-row blocks of the expert's
-// weight matrix, processed one after the other (the index kernel emits single blocks).
+// One work item of the grouped GEMM: one token tile against one kBlockRows-row block of the expert's weight matrix.
 struct __align__(16) WorkItem {
   int expert;  // expert index
-  int ntile;   // first kTileN-row block of that expert's weight matrix
-  int tile;    // global token-tile index (rows tile*kTileM .. of the quantised activations)
+  int ntile;   // kBlockRows-row block of that expert's weight matrix
+  int tile;    // global token-tile index
   int row0;    // first permuted row of the token tile
-  int ntok;    // valid token rows in the tile (1..kTokTile)
-  int nblk;    // row blocks in this item
-  int pad[2];
+  int ntok;    // token rows in the tile (1..kMaxTileTok)
+  int pad[3];
 };
 
 struct GemmArgs {
@@ -89,13 +124,14 @@ struct GemmArgs {
   int K;          // reduction length in elements (multiple of 32)
   int R;          // weight rows per expert on this rank
   int n_kchunks;  // ceil(K / kChunkK)
-  int n_ntiles;   // ceil(R / kTileN)
-  const uint8_t *w_tiles;     // weight tiles [E][n_ntiles][n_kchunks][kWTileStride], see LayerWeights::w1_tiles
-  const uint8_t *sfa;         // activation scales, one 512-byte atom per token tile
-  int sfa_tile_stride;        // bytes between token tiles' atoms (0: one atom shared by all tiles)
+  int n_ntiles;   // ceil(R / kBlockRows)
+  const uint8_t *w_tiles;     // weight tiles [E][n_ntiles][2][n_kchunks * kWTileBytes], see LayerWeights::w1_tiles
+  const uint8_t *xq;          // token rows, e4m3 [tile][slice_pairs(n_kchunks)][kPairBytes] (x_pair_offset)
+  const uint8_t *sfb;         // their scales, kSfbTileBytes per token tile
+  int sfb_tile_stride;        // bytes between token tiles' scales (0: shared by all tiles)
   const __nv_bfloat16 *bias;  // [E][R]
   int add_bias;               // MLP2 on TP ranks other than 0 leaves the bias out
-  uint8_t *hq_out;            // MLP1: quantised SwiGLU output, e4m3 tiles [tile][hq_nkc][128 rows][128 bytes]
+  uint8_t *hq_out;            // MLP1: quantised SwiGLU output, tiled like xq
   int hq_joff, hq_nkc;        //       column of the shard's first output inside MLP2's k window; its k slices
   __half *y_out;              // MLP2: [P, ld_out] fp16
   int ld_out;
@@ -111,14 +147,15 @@ struct MlpFuse {
   int phase_begin, phase_end;
   unsigned int *tile_done;   // [total_slot + 1], zeroed by build_index_kernel; nullptr: phases in separate launches
   int total_slot;            // the last word counts the MLP1 items of all tiles
-  int done_per_tile;         // epilogue warps x MLP1 weight blocks
+  int done_per_tile;         // CTAs of a pair x MLP1 weight blocks
 };
 
 struct LayerWeights {
   bool loaded = false;
-  // MLP1 weights as the GEMM streams them: one 16 KB tile per (expert, 240-row block, 128-wide slice of k),
-  // tiles of a block in k order: [240 rows x 64 bytes of packed e2m1 codes][two 512-byte E8M0 scale atoms in
-  // the order tcgen05.cp wants].  Rows or k beyond the matrix hold zero codes and scale 1 (byte 127).
+  // MLP1 weights as the GEMM streams them, 8 KB per (expert, 240-row block, 120-row half, 128-wide slice of k):
+  // 120 rows x 64 bytes of packed e2m1 codes and one 512-byte E8M0 scale atom in the order tcgen05.cp wants, two
+  // slices stored together (w_codes_offset, w_scales_offset).  Rows or k beyond the matrix hold zero codes and
+  // scale 1 (byte 127).
   uint8_t *w1_tiles = nullptr;
   __nv_bfloat16 *b1 = nullptr;   // [E, R1]
   uint8_t *w2_tiles = nullptr;   // MLP2 weights [E, H, Kw], same tiling
@@ -128,7 +165,8 @@ struct LayerWeights {
   uint8_t *w2_scales_raw = nullptr;  // [E, H, Dl/32]
   __nv_bfloat16 *router_w3 = nullptr;  // [3][E][H] exact 3-way bf16 split of the fp32 router weight
   float *router_b = nullptr;           // [E]
-  CUtensorMap tm_w1, tm_w2, tm_router;
+  CUtensorMap tm_w1[2], tm_w2[2];   // boxes of a pair of k slices, and of the single last one
+  CUtensorMap tm_router;
 };
 
 }  // namespace moe
@@ -142,6 +180,7 @@ struct moe_ctx {
   int joff;       // d0 - k0: column of the shard's first SwiGLU output inside that window
   int max_rows, max_pairs;
   int sm_count;
+  int gemm_grid = 0;        // CTAs of the expert GEMM (two per pair) the device keeps resident at once
   int router_cluster = 0;   // largest thread-block cluster the fused router kernel can use on this device (0: none)
   cudaStream_t stream = nullptr;  // used by moe_forward_host
   std::vector<moe::LayerWeights> layers;
@@ -157,14 +196,14 @@ struct moe_ctx {
   int *offsets = nullptr;           // d_expert_offsets    [E+1]
   int *pair_row = nullptr;          // local_ids_g         [max_rows, K]
   int *row_token = nullptr;         // expert_row_token_g  [max_pairs]
-  int *pair_slot = nullptr;         // row of the high term of (token, k) in xq [max_rows, K]
+  int2 *pair_slot = nullptr;        // place of (token, k) in xq: tile * kMaxTileTok + token, scale row [max_rows, K]
   unsigned int *tile_done = nullptr;   // [max_tiles + 1] MlpFuse::tile_done
   __half *xperm = nullptr;          // expert_input_buffer [max_pairs, H]   fp16 (validation GEMM only)
   __half *hbuf = nullptr;           // gate_up             [max_pairs, Dl]  fp16 (validation GEMM only)
-  uint8_t *xq = nullptr;            // expert_input_buffer as e4m3 high/low rows, [max_tiles][k slices][128 rows][128 B]
+  uint8_t *xq = nullptr;            // expert_input_buffer as e4m3 high/low rows, [max_tiles][pairs of k slices][kPairBytes]
   uint8_t *hq = nullptr;            // gate_up as e4m3 high/low rows, same tiling over MLP2's k window
-  uint8_t *sfa_x = nullptr;         // per-tile scale atoms of xq [max_tiles][512]
-  uint8_t *sfa_h = nullptr;         // the one scale atom of hq   [512]
+  uint8_t *sfb_x = nullptr;         // per-tile scale atoms of xq [max_tiles][1024]
+  uint8_t *sfb_h = nullptr;         // the scale atoms of hq, the same for every tile [1024]
   int *tile_base = nullptr;         // first token tile of each expert [E+1]
   int max_tiles = 0;
   int h_exp = 0;                    // hq holds e4m3(h * 2^-h_exp)
@@ -175,7 +214,6 @@ struct moe_ctx {
   int *n_work = nullptr;            // [2]
   int max_work1 = 0, max_work2 = 0;
   unsigned int *status = nullptr;
-  CUtensorMap tm_x1, tm_x2;
   int last_rows = 0;
   long long launches = 0;
   moe::TpPeers peers = {};          // TP group view; own entries are set at creation
@@ -244,10 +282,10 @@ void launch_topk_softmax(float *logits, const float *partial, int splits, const 
                          int row_offset = 0);
 void launch_count_experts(const int *idx, int n, int E, int *counts, cudaStream_t s);
 void launch_build_index(const int *topk_idx, const int *counts, int T, int E, int K, int n_ntiles1, int n_ntiles2,
-                        int *offsets, int *tile_base, int *pair_row, int *row_token, int *pair_slot, unsigned int *tile_done, int tile_done_total_slot, WorkItem *work1,
+                        int *offsets, int *tile_base, int *pair_row, int *row_token, int2 *pair_slot, unsigned int *tile_done, int tile_done_total_slot, WorkItem *work1,
                         WorkItem *work2, int *n_work, int max_work1, int max_work2, unsigned int *status,
                         cudaStream_t s);
-void launch_quantize_rows(const __nv_bfloat16 *t, const int *pair_slot, int T, int K, uint8_t *xq, uint8_t *sfa, int H,
+void launch_quantize_rows(const __nv_bfloat16 *t, const int2 *pair_slot, int T, int K, uint8_t *xq, uint8_t *sfb, int H,
                           cudaStream_t s);
 int quantize_rows_max_hidden();
 void launch_gather_rows(const __nv_bfloat16 *t, const int *row_token, const int *offsets, int E, __half *xperm,
@@ -260,9 +298,9 @@ void launch_rmsnorm_rows(const __nv_bfloat16 *x, const __nv_bfloat16 *w, __nv_bf
                          cudaStream_t s);
 
 // expert_gemm_sm100.cu
-cudaError_t expert_gemm_init();
-void launch_expert_mlp(const CUtensorMap &tm_w1, const CUtensorMap &tm_x1, const GemmArgs &a, const CUtensorMap &tm_w2,
-                       const CUtensorMap &tm_x2, const GemmArgs &b, const MlpFuse &f, int grid, cudaStream_t s);
+cudaError_t expert_gemm_init(int *grid);   // per-device kernel attributes; call with the device current
+void launch_expert_mlp(const CUtensorMap (&tm_w1)[2], const GemmArgs &a, const CUtensorMap (&tm_w2)[2], const GemmArgs &b,
+                       const MlpFuse &f, int grid, cudaStream_t s);
 int expert_mlp_done_per_tile(int n_ntiles1);
 
 // tp_collectives.cu

@@ -104,7 +104,7 @@ void launch_topk_softmax(float *logits, const float *partial, int splits, const 
 __global__ void __launch_bounds__(1024)
 build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ counts, int T, int E, int K,
                    int n_ntiles1, int n_ntiles2, int *__restrict__ offsets, int *__restrict__ tile_base,
-                   int *__restrict__ pair_row, int *__restrict__ row_token, int *__restrict__ pair_slot,
+                   int *__restrict__ pair_row, int *__restrict__ row_token, int2 *__restrict__ pair_slot,
                    unsigned int *__restrict__ tile_done, int tile_done_total_slot, WorkItem *__restrict__ work1,
                    WorkItem *__restrict__ work2, int *__restrict__ n_work, int max_work1, int max_work2,
                    unsigned int *status) {
@@ -139,7 +139,7 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ cou
   for (int i = tid; i < e; i += blockDim.x) {
     const int c = counts[i];
     my_rows += c;
-    my_tiles += (c + kTokTile - 1) / kTokTile;
+    my_tiles += expert_tiles(c);
   }
 #pragma unroll
   for (int off = 16; off; off >>= 1) {
@@ -157,7 +157,7 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ cou
   int off = 0, tiles_before = 0;
   for (int i = 0; i < n_warps; ++i) { off += s_red[0][i]; tiles_before += s_red[1][i]; }
   const int cnt = counts[e];
-  const int ntt = (cnt + kTokTile - 1) / kTokTile;  // token tiles of this expert (rows e's tiles, in order)
+  const int ntt = expert_tiles(cnt), per_tile = tokens_per_tile(cnt);  // this expert's token tiles
   if (tid == 0) {
     offsets[e] = off;
     tile_base[e] = tiles_before;
@@ -179,8 +179,10 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ cou
       if (pos < cnt) {
         const int r = off + pos;
         row_token[r] = t;
-        // where the row's high term goes in the quantised activations: token tile, then 2 rows per token
-        pair_slot[static_cast<size_t>(t) * K + hit] = (tiles_before + pos / kTokTile) * kTileM + 2 * (pos % kTokTile);
+        // where the row goes in the quantised activations: its tile and place there, and the place of its scales
+        const int tt = pos / per_tile, i = pos - tt * per_tile;
+        pair_slot[static_cast<size_t>(t) * K + hit] =
+            make_int2((tiles_before + tt) * kMaxTileTok + i, x_operand_row(i, tile_n(min(per_tile, cnt - tt * per_tile))));
         pair_row[static_cast<size_t>(t) * K + hit] = r;
       } else {
         atomicOr(status, ST_BAD_INDEX);
@@ -193,11 +195,8 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ cou
   for (int t0 = t_rest; t0 < t_end; t0 += 32) place(t0 + lane, hit_of(t0 + lane));
   if (tid == 0 && total_hits != cnt) atomicOr(status, ST_BAD_INDEX);
 
-  // work items: one per (token tile of kTokTile rows, block of kTileN weight rows); items that share a
-  // weight block are adjacent so that block is fetched from HBM once and re-read from L2.  Single blocks
-  // rather than pairs: the items of a launch are dealt round-robin to one CTA per SM, and the finer the
-  // items, the smaller the idle share of the last round (930 pair items of MLP2 over 148 SMs lose 10 %,
-  // 1860 single ones 3 %).
+  // work items: one per (token tile, block of kBlockRows weight rows); items that share a
+  // weight block are adjacent so that block is fetched from HBM once and re-read from L2.
   for (int which = 0; which < 2; ++which) {
     const int nn = which ? n_ntiles2 : n_ntiles1;
     WorkItem *work = which ? work2 : work1;
@@ -209,10 +208,9 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ cou
       it.expert = e;
       it.ntile = nt;
       it.tile = tiles_before + tt;
-      it.row0 = off + tt * kTokTile;
-      it.ntok = min(kTokTile, cnt - tt * kTokTile);
-      it.nblk = 1;
-      it.pad[0] = it.pad[1] = 0;
+      it.row0 = off + tt * per_tile;
+      it.ntok = min(per_tile, cnt - tt * per_tile);
+      it.pad[0] = it.pad[1] = it.pad[2] = 0;
       if (start + i < cap) work[start + i] = it;
       else atomicOr(status, ST_BAD_INDEX);
     }
@@ -221,7 +219,7 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ cou
 }
 
 void launch_build_index(const int *topk_idx, const int *counts, int T, int E, int K, int n_ntiles1, int n_ntiles2,
-                        int *offsets, int *tile_base, int *pair_row, int *row_token, int *pair_slot,
+                        int *offsets, int *tile_base, int *pair_row, int *row_token, int2 *pair_slot,
                         unsigned int *tile_done, int tile_done_total_slot, WorkItem *work1, WorkItem *work2, int *n_work, int max_work1, int max_work2,
                         unsigned int *status, cudaStream_t s) {
   build_index_kernel<<<E, T > 2048 ? 1024 : 256, 0, s>>>(topk_idx, counts, T, E, K, n_ntiles1, n_ntiles2, offsets, tile_base,
@@ -237,10 +235,9 @@ void launch_build_index(const int *topk_idx, const int *counts, int T, int E, in
 // [128, 256), high = e4m3(x/s) and low = e4m3((x/s - high) * 16).  A bf16 value
 // has 8 significant bits, the high term keeps 4 of them and the residual fits the
 // 4 of the low term, so high + low/16 == x/s exactly unless x is more than 2^13
-// below the row maximum.  Row 2i of a 128-row token tile is the high term of the
-// tile's token i, row 2i+1 the low term; their UE8M0 scales (127+e, 127+e-4) go
-// into the tile's 512-byte scale atom, byte (r%32)*16 + (r/32)*4 + kb for row r
-// and every k block kb (the scale is per row, so the four bytes are equal).
+// below the row maximum.  Where the two rows lie in the token tile: x_pair_offset; their UE8M0 scales
+// (127+e, 127+e-4) go into the tile's 512-byte scale atoms, byte (r%32)*16 + (r/32 %4)*4 + kb of atom r/128 for
+// operand row r and every k block kb (the scale is per row, so the four bytes are equal).
 // ---------------------------------------------------------------------------
 // The two rows depend on the token only, not on the expert, so a warp quantises one TOKEN (its row stays in
 // the warp's registers: kQrVec x 32 bytes per lane) and stores the result once per selected expert, at the
@@ -249,14 +246,14 @@ constexpr int kQrWarps = 4;
 
 template <int kQrVec>         // 6: rows of up to 3072 elements, 8: up to 4096
 __global__ void __launch_bounds__(kQrWarps * 32)
-quantize_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int *__restrict__ pair_slot, int T, int K,
-                     uint8_t *__restrict__ xq, uint8_t *__restrict__ sfa, int H) {
+quantize_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int2 *__restrict__ pair_slot, int T, int K,
+                     uint8_t *__restrict__ xq, uint8_t *__restrict__ sfb, int H) {
   const int lane = threadIdx.x & 31;
   const int tok = blockIdx.x * kQrWarps + (threadIdx.x >> 5);
   if (tok >= T) return;   // whole warps leave: no block-wide barrier below
-  int slot[kMaxTopK];
+  int2 slot[kMaxTopK];
 #pragma unroll
-  for (int k = 0; k < kMaxTopK; ++k) slot[k] = k < K ? pair_slot[static_cast<size_t>(tok) * K + k] : -1;
+  for (int k = 0; k < kMaxTopK; ++k) slot[k] = k < K ? pair_slot[static_cast<size_t>(tok) * K + k] : make_int2(-1, 0);
   const uint4 *src = reinterpret_cast<const uint4 *>(t + static_cast<size_t>(tok) * H);
   const int ngrp = H / 16;    // a lane takes groups of 16 elements: 32 bytes in, 16 + 16 bytes out
   uint4 v[kQrVec][2];
@@ -281,8 +278,8 @@ quantize_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int *__restrict_
   int e = static_cast<int>((__float_as_uint(amax) >> 23) & 0xffu) - 127 - 7;
   e = max(-120, min(e, 120));
   const float inv = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);  // 2^-e
-  // activation tiles: [tile][k slice][128 rows][128 bytes]; 16 elements never straddle a slice
-  const int n_kc = (H + kChunkK - 1) / kChunkK;
+  // activation tiles: see x_pair_offset; 16 elements never straddle a slice
+  const int n_pairs = slice_pairs((H + kChunkK - 1) / kChunkK);
 #pragma unroll
   for (int u = 0; u < kQrVec; ++u) {
     const int g = lane + u * 32;
@@ -314,37 +311,36 @@ quantize_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int *__restrict_
         l8[2 * h + q] = c2 | (d2 << 16);
       }
     }
-    const size_t in_tile = static_cast<size_t>(g >> 3) * (kTileM * kChunkK) + (g & 7) * 16;  // slice g/8, byte 16*(g%8)
 #pragma unroll
     for (int k = 0; k < kMaxTopK; ++k) {
-      if (slot[k] < 0) continue;
-      const int tile = slot[k] / kTileM, i2 = slot[k] % kTileM;   // i2 = 2 * (token's place in the tile)
-      uint8_t *dst = xq + (static_cast<size_t>(tile) * n_kc * kTileM + i2) * kChunkK + in_tile;
-      *reinterpret_cast<uint4 *>(dst) = make_uint4(h8[0], h8[1], h8[2], h8[3]);
-      *reinterpret_cast<uint4 *>(dst + kChunkK) = make_uint4(l8[0], l8[1], l8[2], l8[3]);   // the low row follows
+      if (slot[k].x < 0) continue;
+      const int tile = slot[k].x / kMaxTileTok, i = slot[k].x % kMaxTileTok;
+      uint8_t *dst = xq + (static_cast<size_t>(tile) * n_pairs + (g >> 4)) * kPairBytes;   // 16 groups to a pair of slices
+      *reinterpret_cast<uint4 *>(dst + x_pair_offset(i, 0, (g & 15) * 16)) = make_uint4(h8[0], h8[1], h8[2], h8[3]);
+      *reinterpret_cast<uint4 *>(dst + x_pair_offset(i, 1, (g & 15) * 16)) = make_uint4(l8[0], l8[1], l8[2], l8[3]);
     }
   }
   if (lane < 2) {
     const uint32_t byte = static_cast<uint32_t>(127 + e - 4 * lane);
 #pragma unroll
     for (int k = 0; k < kMaxTopK; ++k) {
-      if (slot[k] < 0) continue;
-      const int tile = slot[k] / kTileM, rr = slot[k] % kTileM + lane;  // row inside the tile: even = high, odd = low
-      uint8_t *atom = sfa + static_cast<size_t>(tile) * kSfAtomBytes;
-      *reinterpret_cast<uint32_t *>(atom + (rr % 32) * 16 + (rr / 32) * 4) = byte * 0x01010101u;
+      if (slot[k].x < 0) continue;
+      const int tile = slot[k].x / kMaxTileTok, rr = slot[k].y + lane;  // operand row: even = high, odd = low
+      uint8_t *atom = sfb + static_cast<size_t>(tile) * kSfbTileBytes + rr / 128 * kSfAtomBytes;
+      *reinterpret_cast<uint32_t *>(atom + (rr % 32) * 16 + (rr / 32 % 4) * 4) = byte * 0x01010101u;
     }
   }
 }
 
 int quantize_rows_max_hidden() { return 32 * 8 * 16; }
 
-void launch_quantize_rows(const __nv_bfloat16 *t, const int *pair_slot, int T, int K, uint8_t *xq, uint8_t *sfa, int H,
+void launch_quantize_rows(const __nv_bfloat16 *t, const int2 *pair_slot, int T, int K, uint8_t *xq, uint8_t *sfb, int H,
                           cudaStream_t s) {
   const int blocks = (T + kQrWarps - 1) / kQrWarps;
   if (H <= 32 * 6 * 16)
-    quantize_rows_kernel<6><<<blocks, kQrWarps * 32, 0, s>>>(t, pair_slot, T, K, xq, sfa, H);
+    quantize_rows_kernel<6><<<blocks, kQrWarps * 32, 0, s>>>(t, pair_slot, T, K, xq, sfb, H);
   else
-    quantize_rows_kernel<8><<<blocks, kQrWarps * 32, 0, s>>>(t, pair_slot, T, K, xq, sfa, H);
+    quantize_rows_kernel<8><<<blocks, kQrWarps * 32, 0, s>>>(t, pair_slot, T, K, xq, sfb, H);
 }
 
 // ---------------------------------------------------------------------------

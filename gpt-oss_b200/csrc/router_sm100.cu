@@ -45,9 +45,6 @@ constexpr int kRtTmemCols = 128;
 constexpr int kRtRedPitch = (kRtExp + 4) * 4;    // bytes per parked accumulator row: 16-byte stores of a warp spread over all banks
 static_assert(kRtTok * kRtRedPitch <= kRtStages * kRtStage, "the parked accumulator reuses the ring");
 
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // kind::f16 with bf16 operands, fp32 accumulator, both operands K-major, M = 128.
 __host__ __device__ constexpr uint32_t idesc_bf16_m128(uint32_t n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);

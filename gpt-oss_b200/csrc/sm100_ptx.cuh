@@ -1,7 +1,6 @@
 // Thin inline-PTX wrappers for the sm_100a features the expert GEMM uses:
 // mbarrier, TMA (cp.async.bulk[.tensor], never with cluster multicast), tensor
-// memory (tcgen05.alloc/ld/st), and the tcgen05.mma instruction with its A operand
-// in tensor memory.  Every wait is bounded: a wait that runs out records a code
+// memory (tcgen05.alloc/ld), and the block-scaled tcgen05.mma of a CTA pair.  Every wait is bounded: a wait that runs out records a code
 // in a status word and returns false so the kernel can unwind (free its tensor
 // memory, leave) instead of hanging the device.
 #pragma once
@@ -43,6 +42,25 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
 }
+// Arrives on the same barrier of CTA `cta` of the cluster.  Default semantics on purpose: what the arrival
+// publishes here are copies that the copy engine has completed and tensor-memory loads that have returned, no
+// ordinary stores of this thread, and a release at cluster scope is a memory barrier that costs ~0.9 us.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, uint32_t cta) {
+  asm volatile(
+      "{\n\t.reg .b32 r;\n\t"
+      "mapa.shared::cluster.u32 r, %0, %1;\n\t"
+      "mbarrier.arrive.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar), "r"(cta)
+      : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// All threads of all CTAs of the cluster.
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -54,7 +72,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-
 // Bounded wait.  `abort_flag` is a CTA-shared word that any role sets when it
 // gives up; `status` is the global status word the host reads.  About one
 // second of polling at most, and it leaves early once another role aborted.
@@ -134,6 +151,14 @@ __device__ __forceinline__ void tma_load_3d_hint(uint32_t dst, const CUtensorMap
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y), "r"(z), "l"(policy)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_5d_hint(uint32_t dst, const CUtensorMap *m, int x, int y, int z, int u, int v,
+                                                 uint32_t bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%3, %4, %5, %6, %7}], [%2], %8;"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(u), "r"(v), "l"(policy)
+      : "memory");
+}
 __device__ __forceinline__ void bulk_load_hint(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar,
                                                uint64_t policy) {
   asm volatile(
@@ -161,6 +186,16 @@ __device__ __forceinline__ void tmem_relinquish() {
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
+// The same for a pair of CTAs (cta_group::2): one warp of each CTA executes them, the space is the same in both.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
@@ -168,7 +203,6 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // One warp, 32 lanes x 16 consecutive 32-bit columns; lane i <-> TMEM lane
 // (taddr.lane + i).  A warp may only touch lanes 32*(warp_id % 4) .. +31.
@@ -181,27 +215,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-      "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-      : "memory");
-}
-
 // ---------------------------------------------------------------- tcgen05.mma
-// D[tmem] (+)= A[tmem] * B[smem]^T, kind::f16 (fp16 operands, fp32 accumulate),
-// M = 128, K = 16 per instruction, issued by ONE thread.
-__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // Arrives (count 1) on an mbarrier once every MMA issued so far by this thread
 // has completed.  Implies tcgen05.fence::before_thread_sync.
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
@@ -209,68 +223,67 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
                : "memory");
 }
 
-// Instruction descriptor, kind::f16: fp32 accumulator, fp16 A and B, both
-// K-major, M = 128, N = n (multiple of 16, 16..256).
-__host__ __device__ constexpr uint32_t idesc_f16_m128(uint32_t n) {
-  return (1u << 4)            // D format  = F32
-         | (0u << 7)          // A format  = F16
-         | (0u << 10)         // B format  = F16
-         | ((n >> 3) << 17)   // N >> 3
-         | ((128u >> 4) << 24);  // M >> 4
+// The same for the MMAs of a CTA pair, arriving on the barrier at this offset in both CTAs.
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+      "h"(static_cast<uint16_t>(3))
+      : "memory");
 }
 
 // Shared-memory matrix descriptor of a K-major operand stored as rows of 128
 // bytes with the 128-byte swizzle (what a TMA box of 64 fp16 x rows with
-// CU_TENSOR_MAP_SWIZZLE_128B writes): 8-row groups are 1024 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
+// CU_TENSOR_MAP_SWIZZLE_128B writes): 8-row groups are group_bytes apart (1024 when they are adjacent).
+__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr, uint32_t group_bytes = 1024) {
   uint64_t d = 0;
   d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);  // start address
   d |= static_cast<uint64_t>(1) << 16;                  // leading byte offset (unused with swizzle)
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;          // stride byte offset
+  d |= static_cast<uint64_t>(group_bytes >> 4) << 32;   // stride byte offset
   d |= static_cast<uint64_t>(1) << 46;                  // descriptor version of sm_100
   d |= static_cast<uint64_t>(2) << 61;                  // SWIZZLE_128B
   return d;
 }
 
-// D[tmem] (+)= (A * SFA) * (B * SFB)^T, kind::mxf8f6f4 with one UE8M0 scale per 32
-// elements of K for every row of A and of B; A and B from shared memory, scale
-// factors from tensor memory, M = 128, K = 32 per instruction.
-__device__ __forceinline__ void mma_mxf8f6f4_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                uint32_t accumulate, uint32_t sfa_tmem, uint32_t sfb_tmem) {
+// D[tmem] (+)= (A * SFA) * (B * SFB)^T over a CTA pair, kind::mxf8f6f4 with one UE8M0 scale per 32 elements of K
+// for every row of A and of B; M = 256 (128 rows in each CTA's shared memory, accumulated in its tensor memory),
+// N (the first N/2 rows of B in the even CTA's shared memory, the others in the odd one's), K = 32.  Scale factors
+// from tensor memory: each CTA holds those of its A rows and of all N rows of B.
+__device__ __forceinline__ void mma_mxf8f6f4_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                  uint32_t accumulate, uint32_t sfa_tmem, uint32_t sfb_tmem) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
+      "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem)
       : "memory");
 }
 
-// Instruction descriptor, kind::mxf8f6f4 block scaled: A = e4m3, B = e2m1 (4-bit
-// codes in 8-bit containers as the 16U4_ALIGN16B tensor map writes them), both
-// K-major, UE8M0 scales, M = 128, N = n.  sf_id selects which of the four scale
-// bytes of a tensor-memory column (which 32-wide k block of a 128-wide slice)
-// the instruction applies, for A and for B.
-__host__ __device__ constexpr uint32_t idesc_mxf8f6f4_m128(uint32_t n, uint32_t sf_id) {
-  return (sf_id << 4)          // B scale-factor id
-         | (0u << 7)           // A format = E4M3
-         | (5u << 10)          // B format = E2M1
+// Instruction descriptor, kind::mxf8f6f4 block scaled: A = e2m1 (4-bit codes in 8-bit containers as the
+// 16U4_ALIGN16B tensor map writes them), B = e4m3, both K-major, UE8M0 scales, M = 256, N = n (multiple of 16).
+// sf_id selects which of the four scale bytes of a tensor-memory column (which 32-wide k block of a 128-wide
+// slice) the instruction applies, for A and for B.
+__host__ __device__ constexpr uint32_t idesc_sf_id(uint32_t sf_id) { return (sf_id << 4) | (sf_id << 29); }
+__host__ __device__ constexpr uint32_t idesc_mxf8f6f4_m256(uint32_t n, uint32_t sf_id) {
+  return idesc_sf_id(sf_id)
+         | (5u << 7)           // A format = E2M1
+         | (0u << 10)          // B format = E4M3
          | ((n >> 3) << 17)    // N >> 3
          | (1u << 23)          // scale format = UE8M0
-         | ((128u >> 4) << 24) // M >> 4
-         | (sf_id << 29);      // A scale-factor id
+         | ((256u >> 4) << 24);  // M >> 4
 }
 
 // Copies one 512-byte scale-factor atom (32 rows x 16 bytes, no swizzle) from
 // shared memory into 4 tensor-memory columns, replicated into all four 32-lane
-// quadrants.  Byte (r % 32) * 16 + (r / 32) * 4 + kb of the atom is the scale of
+// quadrants, in both CTAs of the pair (each from its own shared memory).  Byte
+// (r % 32) * 16 + (r / 32) * 4 + kb of the atom is the scale of
 // row r, k block kb.  Issued by one thread; ordered before later tcgen05.mma of
 // the same thread.
-__device__ __forceinline__ void tmem_cp_sf_atom(uint32_t taddr, uint32_t saddr) {
+__device__ __forceinline__ void tmem_cp_sf_atom_pair(uint32_t taddr, uint32_t saddr) {
   uint64_t d = 0;
   d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);  // start address
   d |= static_cast<uint64_t>(128 >> 4) << 32;           // stride between 8-row groups: 8 x 16 bytes
   d |= static_cast<uint64_t>(1) << 46;                  // descriptor version of sm_100
-  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(d) : "memory");
+  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(d) : "memory");
 }
 
 // ---------------------------------------------------------------- MXFP4 decode

@@ -13,7 +13,7 @@ namespace moe {
 __device__ __forceinline__ float swiglu_clamped(float gate, float up, float limit, float alpha) {
   gate = fminf(gate, limit);
   up = fminf(fmaxf(up, -limit), limit);
-  const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(__fmul_rn(-alpha, gate))));
+  const float sig = __frcp_rn(__fadd_rn(1.0f, expf(__fmul_rn(-alpha, gate))));   // the division 1 / x, correctly rounded
   return __fmul_rn(__fmul_rn(gate, sig), __fadd_rn(up, 1.0f));
 }
 

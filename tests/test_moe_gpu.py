@@ -551,3 +551,21 @@ def test_expert_output_beyond_fp16_is_reported(pkg, synth):
         assert np.array_equal(blk.forward_host(0, tokens), good)
     finally:
         blk.close()
+
+
+# Tokens of one expert at the edges of the expert GEMM's token tiles (steps of 8 tokens, 96 to a tile, tiles of equal
+# size) and k slices (one, an odd and an even number of 128-wide slices, with and without a tail; weight rows that
+# do not fill a 240-row block).  With as many experts as selections every expert gets every token.
+@pytest.mark.parametrize("H,D", [(64, 32), (128, 160), (288, 256), (416, 288)])
+@pytest.mark.parametrize("T", [1, 4, 5, 8, 9, 95, 96, 97, 192, 193, 289])
+def test_token_tile_and_slice_edges(T, H, D, pkg, synth, port):
+    layer = synth.make_layer(4, H, D, seed=11 * H + D)
+    tokens = synth.make_tokens(T, H, seed=T)
+    ref = port.moe_layer(layer, tokens)
+    blk, out = run_block(pkg, layer, tokens)
+    try:
+        assert (blk.debug(pkg.DBG_COUNTS) == T).all()
+        same = check_selection(blk.debug(pkg.DBG_TOPK_IDX), ref[1], ref[0])
+        check_output(out, blk.debug(pkg.DBG_OUT_F32), ref[3], synth, rows=same, label=f"T{T} H{H} D{D}")
+    finally:
+        blk.close()
