@@ -115,7 +115,8 @@ struct __align__(16) WorkItem {
   int tile;    // global token-tile index
   int row0;    // first permuted row of the token tile
   int ntok;    // token rows in the tile (1..kMaxTileTok)
-  int pad[3];
+  int lead;    // 1 for the first of the items that share a weight block: it brings the block into L2
+  int pad[2];
 };
 
 struct GemmArgs {

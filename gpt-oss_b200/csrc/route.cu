@@ -210,7 +210,8 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ cou
       it.tile = tiles_before + tt;
       it.row0 = off + tt * per_tile;
       it.ntok = min(per_tile, cnt - tt * per_tile);
-      it.pad[0] = it.pad[1] = it.pad[2] = 0;
+      it.lead = tt == 0;
+      it.pad[0] = it.pad[1] = 0;
       if (start + i < cap) work[start + i] = it;
       else atomicOr(status, ST_BAD_INDEX);
     }
