@@ -9,9 +9,9 @@
 // scan of the 16 table entries.
 //
 // Four lanes per 32-element block (the reference gives it a "logical warp" of
-// 32), shuffles instead of its shared-memory staging, thresholds instead of its
-// 16-way scan, a multiplication by 2^-exp instead of its division; a grid-stride
-// loop over the blocks of the call.  HBM-bound: 4 bytes read and 17/32 byte written per
+// 32), shuffles instead of its shared-memory staging, the conversion instruction
+// (thresholds where it rounds differently) instead of its 16-way scan, a multiplication
+// by 2^-exp instead of its division; a grid-stride loop over the blocks of the call.  HBM-bound: 4 bytes read and 17/32 byte written per
 // element.
 #include <cstdarg>
 #include <cstdio>
@@ -33,7 +33,68 @@ __device__ __forceinline__ uint32_t e2m1_first_nearest(float x) {
   return (x < 0.f && idx != 0) ? (idx | 8u) : idx;
 }
 
-// Four lanes per 32-element block, eight consecutive elements per lane (two 16-byte loads in flight).
+// Eight values (already divided by the block scale) -> eight codes by the conversion instruction, which rounds to the
+// nearest magnitude, saturates at 6, and differs from the scan above in two ways.  At an exact midpoint it takes the
+// even code, which can be the larger magnitude: the caller passes values there a last place closer to zero.  A
+// negative value that rounds to zero keeps its sign, which the code of the reference does not have: cleared here.
+__device__ __forceinline__ uint32_t e2m1x8_nearest(const float (&x)[8]) {
+  uint32_t word;
+  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
+      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
+      : "=r"(word)
+      : "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]), "f"(x[4]), "f"(x[5]), "f"(x[6]), "f"(x[7]));
+  const uint32_t nonzero = (word | (word >> 1) | (word >> 2)) & 0x11111111u;
+  return word & (0x77777777u | (nonzero << 3));
+}
+
+// One 32-element block's lane: eight values and the block's largest magnitude -> code word and scale exponent.
+__device__ __forceinline__ uint32_t quantize8(const float (&v)[8], float maxabs, int &exp_scale) {
+  // exp = ilogb(maxabs) - 2 (the largest power of two among the E2M1 magnitudes is 2^2), 0 for a zero block
+  const uint32_t mbits = __float_as_uint(maxabs);
+  exp_scale = 0;
+  float x[8];
+  if (mbits >= 0x01800000u && mbits < 0x7f800000u) {
+    // maximum of at least 2^-124: the exponent field is ilogb, and 2^-exp is a normal float, so multiplying
+    // by it rounds exactly as the reference's division by 2^exp does
+    exp_scale = static_cast<int>(mbits >> 23) - 127 - 2;
+    const float inv = __uint_as_float(static_cast<uint32_t>(127 - exp_scale) << 23);
+    // Midpoints have at most two bits after the leading one.  A value with nothing in its last 21 bits is scaled by
+    // the next float below 2^-exp, which takes it a last place towards zero: a midpoint then rounds down, anything else
+    // with so few bits is a magnitude of the table or clear of the midpoints and rounds as before.
+    const float inv_below = __uint_as_float(__float_as_uint(inv) - 1u);
+    float sum = 0.f;   // NaN if one of the values is (the others are below 8)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      x[j] = v[j] * ((__float_as_uint(v[j]) & 0x1fffffu) == 0u ? inv_below : inv);
+      sum += x[j];
+    }
+    if (sum == sum) return e2m1x8_nearest(x);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = v[j] * inv;
+  } else {
+    if (maxabs > 0.f) {  // tiny or infinite maximum: the reference's own library calls
+      int e;
+      frexpf(maxabs, &e);
+      exp_scale = (e - 1) - 2;
+    }
+    const float X = ldexpf(1.0f, exp_scale);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = v[j] / X;
+  }
+  uint32_t word = 0;  // low nibble = even element
+#pragma unroll
+  for (int j = 0; j < 8; ++j) word |= e2m1_first_nearest(x[j]) << (4 * j);
+  return word;
+}
+
+// Four lanes per 32-element block, eight consecutive elements per lane, the loads of two groups in flight.  With
+// thresholds an element cost ~25 instructions, 97 us of issue slots at 132.7 M values, and they were the bound; with the
+// conversion instruction ~8, and HBM is: 166 -> 108 us (3.62 -> 5.57 TB/s read and written).
+constexpr int kQuantUnroll = 2;
 __global__ void __launch_bounds__(256)
 mxfp4_quantize_kernel(const float *__restrict__ src, size_t n, uint8_t *__restrict__ codes,
                       uint8_t *__restrict__ scales, size_t n_blocks) {
@@ -41,55 +102,43 @@ mxfp4_quantize_kernel(const float *__restrict__ src, size_t n, uint8_t *__restri
   const size_t total = n_blocks * 4;  // 8-element groups, the last block padded with zeros
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   const bool vec_ok = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
-  for (size_t base = static_cast<size_t>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31); base < total; base += stride) {
-    const size_t q = base + lane, g0 = q * 8;
-    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // elements past the end count as 0 (mxfp4.hpp:170-174)
-    if (q < total) {
-      if (vec_ok && g0 + 7 < n) {
-        const float4 f0 = __ldg(reinterpret_cast<const float4 *>(src + g0));
-        const float4 f1 = __ldg(reinterpret_cast<const float4 *>(src + g0) + 1);
-        v[0] = f0.x; v[1] = f0.y; v[2] = f0.z; v[3] = f0.w;
-        v[4] = f1.x; v[5] = f1.y; v[6] = f1.z; v[7] = f1.w;
-      } else {
+  for (size_t base = static_cast<size_t>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31); base < total;
+       base += kQuantUnroll * stride) {
+    float v[kQuantUnroll][8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (g0 + j < n) v[j] = src[g0 + j];
+    for (int u = 0; u < kQuantUnroll; ++u) {
+      const size_t q = base + u * stride + lane, g0 = q * 8;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[u][j] = 0.f;   // elements past the end count as 0 (mxfp4.hpp:170-174)
+      if (q < total) {
+        if (vec_ok && g0 + 7 < n) {
+          const float4 f0 = __ldcs(reinterpret_cast<const float4 *>(src + g0));
+          const float4 f1 = __ldcs(reinterpret_cast<const float4 *>(src + g0) + 1);
+          v[u][0] = f0.x; v[u][1] = f0.y; v[u][2] = f0.z; v[u][3] = f0.w;
+          v[u][4] = f1.x; v[u][5] = f1.y; v[u][6] = f1.z; v[u][7] = f1.w;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (g0 + j < n) v[u][j] = src[g0 + j];
+        }
       }
     }
-    // largest |v| of the block; a NaN never wins a '>' in the reference's scan, fmaxf drops it the same way
-    float maxabs = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) maxabs = fmaxf(maxabs, fabsf(v[j]));
-    maxabs = fmaxf(maxabs, __shfl_xor_sync(0xffffffffu, maxabs, 1));
-    maxabs = fmaxf(maxabs, __shfl_xor_sync(0xffffffffu, maxabs, 2));
-    // exp = ilogb(maxabs) - 2 (the largest power of two among the E2M1 magnitudes is 2^2), 0 for a zero block
-    const uint32_t mbits = __float_as_uint(maxabs);
-    int exp_scale = 0;
-    float x[8];
-    if (mbits >= 0x01800000u && mbits < 0x7f800000u) {
-      // maximum of at least 2^-124: the exponent field is ilogb, and 2^-exp is a normal float, so multiplying
-      // by it rounds exactly as the reference's division by 2^exp does
-      exp_scale = static_cast<int>(mbits >> 23) - 127 - 2;
-      const float inv = __uint_as_float(static_cast<uint32_t>(127 - exp_scale) << 23);
+    for (int u = 0; u < kQuantUnroll; ++u) {
+      const size_t q = base + u * stride + lane;
+      // largest |v| of the block; a NaN never wins a '>' in the reference's scan, fmaxf drops it the same way
+      float maxabs = 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) x[j] = v[j] * inv;
-    } else {
-      if (maxabs > 0.f) {  // tiny or infinite maximum: the reference's own library calls
-        int e;
-        frexpf(maxabs, &e);
-        exp_scale = (e - 1) - 2;
+      for (int j = 0; j < 8; ++j) maxabs = fmaxf(maxabs, fabsf(v[u][j]));
+      maxabs = fmaxf(maxabs, __shfl_xor_sync(0xffffffffu, maxabs, 1));
+      maxabs = fmaxf(maxabs, __shfl_xor_sync(0xffffffffu, maxabs, 2));
+      int exp_scale;
+      const uint32_t word = quantize8(v[u], maxabs, exp_scale);
+      if (q < total) {
+        const size_t b = q >> 2;
+        reinterpret_cast<uint32_t *>(codes + b * 16)[q & 3] = word;
+        if ((q & 3) == 0) scales[b] = static_cast<uint8_t>(min(max(exp_scale + 127, 0), 255));
       }
-      const float X = ldexpf(1.0f, exp_scale);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) x[j] = v[j] / X;
-    }
-    uint32_t word = 0;  // low nibble = even element
-#pragma unroll
-    for (int j = 0; j < 8; ++j) word |= e2m1_first_nearest(x[j]) << (4 * j);
-    if (q < total) {
-      const size_t b = q >> 2;
-      reinterpret_cast<uint32_t *>(codes + b * 16)[q & 3] = word;
-      if ((q & 3) == 0) scales[b] = static_cast<uint8_t>(min(max(exp_scale + 127, 0), 255));
     }
   }
 }

@@ -40,6 +40,37 @@ def test_quantizer_matches_oracle(n, pkg, port):
     assert np.array_equal(gs, ps) and np.array_equal(gc, pc)
 
 
+@pytest.mark.parametrize("src_offset", [0, 1])
+def test_quantizer_midpoints_and_neighbours(src_offset, pkg, port):
+    """Every magnitude and midpoint of the table, one and two last places to either side, both signs, under block
+    maxima of several exponents (the smallest ones on the library-call path), zeros and NaN between them."""
+    grid = np.array([0.0, 0.125, 0.25, 0.5, 0.75, 1.0, 1.25, 1.5, 1.75, 2.0, 2.5, 3.0, 3.5, 4.0, 5.0, 6.0, 7.0],
+                    dtype=np.float32)
+    near = np.concatenate([grid, np.nextafter(grid, np.float32(9)), np.nextafter(grid, np.float32(-9)),
+                           np.nextafter(np.nextafter(grid, np.float32(9)), np.float32(9))])
+    near = np.concatenate([near, -near])
+    blocks = []
+    for e in (-126, -125, -122, -60, -7, 0, 30, 120):
+        for i in range(0, len(near), 30):
+            b = np.zeros(32, np.float32)
+            part = near[i:i + 30]
+            b[1:1 + len(part)] = part
+            b[0] = 4.0 if i % 60 else -7.9375      # sets the block's exponent
+            b[31] = np.nan if i == 30 else 0.0
+            blocks.append(b * np.float32(2.0) ** np.float32(e))
+    v = np.concatenate([np.zeros(src_offset, np.float32)] + blocks)[src_offset:]
+    pc, ps = port.quantize(v)
+    import torch
+    d_v = torch.zeros(v.size + src_offset, dtype=torch.float32, device="cuda")
+    d_v[src_offset:] = torch.from_numpy(v).cuda()   # offset 1: the scalar-load path
+    d_c = torch.empty(v.size // 2, dtype=torch.uint8, device="cuda")
+    d_s = torch.empty(v.size // 32, dtype=torch.uint8, device="cuda")
+    pkg.quantize_mxfp4(d_v[src_offset:].data_ptr(), v.size, d_c.data_ptr(), d_s.data_ptr(),
+                       torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert np.array_equal(d_s.cpu().numpy(), ps) and np.array_equal(d_c.cpu().numpy(), pc)
+
+
 def test_quantizer_full_size_properties(pkg, synth, port):
     """One expert's MLP1 matrix at full size (5760 x 2880 fp32, 66 MB): quantising the exact decode of
     MXFP4 weights gives back values that decode to the same floats (a block whose largest code is 3 or
