@@ -172,6 +172,7 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
   cluster_sync_all();   // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dep_sync();   // from here on the work lists and the token rows are read
 
   // Items of a phase are dealt round-robin to the pairs.  In a fused launch the MLP2 deal starts where the MLP1
   // deal ended, so that the pairs with one MLP1 item more are not also the ones with one MLP2 item more.
@@ -546,8 +547,8 @@ cudaError_t expert_gemm_init(int *grid) {
 // Phases [f.phase_begin, f.phase_end) of the expert MLP in one launch: both in the usual call, one at a
 // time (two launches, f.tile_done = nullptr) on request.
 void launch_expert_mlp(const CUtensorMap (&tm_w1)[2], const GemmArgs &a, const CUtensorMap (&tm_w2)[2], const GemmArgs &b,
-                       const MlpFuse &f, int grid, cudaStream_t s) {
-  expert_gemm_kernel<<<grid, kThreads, kSmemBytes, s>>>(tm_w1[0], tm_w1[1], tm_w2[0], tm_w2[1], a, b, f);
+                       const MlpFuse &f, int grid, cudaStream_t s, bool chained) {
+  launch_kernel(expert_gemm_kernel, dim3(grid), kThreads, kSmemBytes, s, chained, 0, tm_w1[0], tm_w1[1], tm_w2[0], tm_w2[1], a, b, f);
 }
 
 int expert_mlp_done_per_tile(int n_ntiles1) { return 2 * n_ntiles1; }

@@ -136,7 +136,11 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
   const int T = rows, P = rows * c->K, E = c->E, H = c->H, K = c->K;
   const int n_nt1 = (c->R1 + kBlockRows - 1) / kBlockRows, n_nt2 = (H + kBlockRows - 1) / kBlockRows;
 
-  CU_TRY(c, cudaMemsetAsync(c->counts, 0, sizeof(int) * E, s));
+  // The kernels of a one-GPU call are chained by programmatic dependent launch; a profile's events between them, and the
+  // side stream and hand-shakes of a group's call, want ordinary launches.
+  const bool chained = !tpcall && !c->profiling;
+  if (c->hist_dirty) CU_TRY(c, cudaMemsetAsync(c->hist, 0, sizeof(int) * E, s));
+  c->hist_dirty = true;
   auto mark = [&]() {
     if (!c->profiling) return;
     cudaEvent_t ev;
@@ -152,7 +156,7 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
   };
   mark();
   if (norm_gain != nullptr && !tpcall) {   // step 0 of moe_gpu on one GPU: t = rmsnorm(x) * gain
-    launch_rmsnorm_rows(residual, norm_gain, c->t_norm, rows, H, s);
+    launch_rmsnorm_rows(residual, norm_gain, c->t_norm, rows, H, s, chained);
     t = c->t_norm;
     c->launches += 1;
   }
@@ -165,19 +169,19 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
     RouteOut ro = {};
     ro.logits = c->logits; ro.bias = w.router_b; ro.K = K;
     if (tpcall) { ro.tp = tp; ro.peers = c->peers; ro.row_offset = rank * tp_rows_local; }
-    else { ro.idx = c->topk_idx; ro.w = c->topk_w; ro.counts = c->counts; }
+    else { ro.idx = c->topk_idx; ro.w = c->topk_w; ro.counts = c->hist; }
     bool ok;
     if (slices > 0) {
-      ok = launch_router_fused(src, w.tm_router, n, H, E, slices, ro, status, s);
+      ok = launch_router_fused(src, w.tm_router, n, H, E, slices, ro, status, s, chained);
       routed_in_one_launch = true;
       mark();
       c->launches -= 1;   // one launch where the tally below counts two
     } else {
       const int splits = router_splits(n, H, c->sm_count);
-      ok = launch_router_partials(src, w.tm_router, c->router_part, n, H, E, splits, status, s);
+      ok = launch_router_partials(src, w.tm_router, c->router_part, n, H, E, splits, status, s, chained);
       mark();
       launch_topk_softmax(ro.logits, c->router_part, splits, ro.bias, n, E, K, ro.idx, ro.w, ro.counts, s, ro.tp,
-                          &ro.peers, ro.row_offset);
+                          &ro.peers, ro.row_offset, chained);
     }
     if (!ok) return fail(c, MOE_ERR_INVALID, "router launch refused (input rows 16-byte aligned, hidden_dim a multiple of 8?)");
     return MOE_OK;
@@ -200,7 +204,7 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
     CU_TRY(c, cudaStreamWaitEvent(c->aux_stream, c->ev_fork, 0));
     push_rows(0, part_a);
     if (norm_gain != nullptr) {   // moe_block: the rows the router reads are normalised here, the push normalises on the fly
-      launch_rmsnorm_rows(residual, norm_gain, c->t_norm, tp_rows_local, H, s);
+      launch_rmsnorm_rows(residual, norm_gain, c->t_norm, tp_rows_local, H, s, false);
       c->launches += 1;
     }
     if (int rc = route_rows(norm_gain != nullptr ? c->t_norm : t_local, tp_rows_local)) return rc;
@@ -212,20 +216,20 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
       c->launches += 1;
     }
     CU_TRY(c, cudaEventRecord(c->ev_join, c->aux_stream));
-    launch_count_experts(c->topk_idx, T * K, E, c->counts, s);
+    launch_count_experts(c->topk_idx, T * K, E, c->hist, s);
     mark();
     c->launches += 4;
   }
-  launch_build_index(c->topk_idx, c->counts, T, E, K, n_nt1, n_nt2, c->offsets, c->tile_base, c->pair_row,
+  launch_build_index(c->topk_idx, c->hist, c->counts, T, E, K, n_nt1, n_nt2, c->offsets, c->tile_base, c->pair_row,
                      c->row_token, c->pair_slot, c->tile_done, c->max_tiles, c->work1, c->work2, c->n_work, c->max_work1,
-                     c->max_work2, status, s);
+                     c->max_work2, status, s, chained);
   if (tpcall) {   // now the gathered rows: this rank's push is complete (side stream), then every peer's
     CU_TRY(c, cudaStreamWaitEvent(s, c->ev_join, 0));
     launch_tp_signal_wait(c->peers, c->tp_flags, tp, rank, kTpPhaseGather, c->tp_epoch, status, s);
   }
   mark();
   if (flags & MOE_FWD_SIMT_GEMM) launch_gather_rows(t, c->row_token, c->offsets, E, c->xperm, H, P, s);
-  else launch_quantize_rows(t, c->pair_slot, T, K, c->xq, c->sfb_x, H, s);
+  else launch_quantize_rows(t, c->pair_slot, T, K, c->xq, c->sfb_x, H, s, chained);
   mark();
   const int add_b2 = c->cfg.tp_rank == 0 ? 1 : 0;
   bool mlp_in_one_launch = false;
@@ -253,13 +257,13 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
     fuse.done_per_tile = expert_mlp_done_per_tile(n_nt1);
     if (flags & MOE_FWD_SPLIT_MLP) {   // MLP1 and MLP2 as two launches
       fuse.phase_begin = 0; fuse.phase_end = 1; fuse.tile_done = nullptr;
-      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, fuse, c->gemm_grid, s);
+      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, fuse, c->gemm_grid, s, chained);
       mark();
       fuse.phase_begin = 1; fuse.phase_end = 2;
-      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, fuse, c->gemm_grid, s);
+      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, fuse, c->gemm_grid, s, chained);
     } else {                           // one launch; the MLP2 stage of a profile is then empty
       fuse.phase_begin = 0; fuse.phase_end = 2; fuse.tile_done = c->tile_done;
-      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, fuse, c->gemm_grid, s);
+      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, fuse, c->gemm_grid, s, chained);
       mark();
       c->launches -= 1;
       mlp_in_one_launch = true;
@@ -270,12 +274,12 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
     const bool partial = (flags & MOE_FWD_PARTIAL_F32) != 0;
     const bool keep_f32 = partial || (c->cfg.flags & MOE_CFG_KEEP_F32_OUT);
     launch_combine(c->ybuf, c->topk_idx, c->topk_w, c->pair_row, T, H, K, partial ? nullptr : out_dev,
-                   keep_f32 ? c->out_f32 : nullptr, s, 0, nullptr, 0, 0, residual);
+                   keep_f32 ? c->out_f32 : nullptr, c->hist, E, s, chained, 0, nullptr, 0, 0, residual);
     mark();
   } else {
     // send half of the reduce-scatter inside the combine; then wait for every peer's rows and add the slots
     launch_combine(c->ybuf, c->topk_idx, c->topk_w, c->pair_row, T, H, K, c->tp_partial,
-                   (c->cfg.flags & MOE_CFG_KEEP_F32_OUT) ? c->out_f32 : nullptr, s, tp, &c->peers, tp_rows_local, rank);
+                   (c->cfg.flags & MOE_CFG_KEEP_F32_OUT) ? c->out_f32 : nullptr, c->hist, E, s, false, tp, &c->peers, tp_rows_local, rank);
     ++c->tp_epoch_rs;
     launch_tp_signal_wait(c->peers, c->tp_flags, tp, rank, kTpPhaseScatter, c->tp_epoch_rs, status, s);
     launch_tp_sum_slots(c->tp_partial, tp, tp_rows_local, H, out_dev, c->sm_count, s, residual);
@@ -285,6 +289,7 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
   c->launches += 7;
   c->last_rows = rows;
   CU_TRY(c, cudaGetLastError());
+  c->hist_dirty = false;
   return MOE_OK;
 }
 
@@ -372,6 +377,8 @@ int moe_create(const moe_config *cfg, moe_handle *out) {
   if ((rc = dev_alloc(c, &c->router_part, std::max<size_t>(T, 128 * static_cast<size_t>(c->sm_count) + 128) * c->E))) return rc;
   if ((rc = dev_alloc(c, &c->topk_idx, T * c->K))) return rc;
   if ((rc = dev_alloc(c, &c->topk_w, T * c->K))) return rc;
+  if ((rc = dev_alloc(c, &c->hist, (size_t)c->E))) return rc;
+  CU_TRY(c, cudaMemset(c->hist, 0, sizeof(int) * c->E));
   if ((rc = dev_alloc(c, &c->counts, (size_t)c->E))) return rc;
   if ((rc = dev_alloc(c, &c->offsets, (size_t)c->E + 1))) return rc;
   if ((rc = dev_alloc(c, &c->pair_row, T * c->K))) return rc;
@@ -459,7 +466,7 @@ int moe_destroy(moe_handle c) {
   for (auto &w : c->layers) free_layer(w);
   for (cudaEvent_t e : c->prof_events) if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : c->prof_pool) cudaEventDestroy(e);
-  cudaFree(c->t_in); cudaFree(c->t_norm); cudaFree(c->logits); cudaFree(c->router_part); cudaFree(c->topk_idx); cudaFree(c->topk_w); cudaFree(c->counts);
+  cudaFree(c->t_in); cudaFree(c->t_norm); cudaFree(c->logits); cudaFree(c->router_part); cudaFree(c->topk_idx); cudaFree(c->topk_w); cudaFree(c->hist); cudaFree(c->counts);
   cudaFree(c->offsets); cudaFree(c->pair_row); cudaFree(c->row_token); cudaFree(c->pair_slot); cudaFree(c->tile_done); cudaFree(c->xperm); cudaFree(c->hbuf);
   cudaFree(c->ybuf); cudaFree(c->out_f32); cudaFree(c->out_bf16); cudaFree(c->work1); cudaFree(c->work2);
   cudaFree(c->n_work); cudaFree(c->status);

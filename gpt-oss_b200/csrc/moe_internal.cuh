@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/moe_b200.h"
@@ -193,7 +194,9 @@ struct moe_ctx {
   float *router_part = nullptr;     // split-k partial sums of the router [splits, rows, E]
   int *topk_idx = nullptr;          // topk_i_g            [max_rows, K]
   float *topk_w = nullptr;          // topk_v_g            [max_rows, K]
-  int *counts = nullptr;            // d_expert_counts     [E]
+  int *hist = nullptr;              // selections per expert of the running call [E]; zero between calls (combine clears it)
+  bool hist_dirty = false;          // a call did not get as far as clearing it
+  int *counts = nullptr;            // d_expert_counts     [E]   hist of the last call, kept
   int *offsets = nullptr;           // d_expert_offsets    [E+1]
   int *pair_row = nullptr;          // local_ids_g         [max_rows, K]
   int *row_token = nullptr;         // expert_row_token_g  [max_pairs]
@@ -253,6 +256,44 @@ inline TensorMapEncodeFn tensor_map_encoder() {
   return fn;
 }
 
+// Programmatic dependent launch.  The kernels of a block run one after the other and the small ones are mostly launch
+// latency and set-up; launched with chained = true a kernel may start while its predecessor in the stream still runs.
+// Every kernel of the chain therefore begins with grid_dep_sync(): it lets the successor start in turn, and waits until
+// the predecessor has completed and its writes are visible.  Before it only parameters, barriers and tensor memory
+// are touched (the router also fetches its weights).  Since every grid waits for the one before it, a completed grid
+// means that all earlier ones are complete.  Without the attribute the wait returns at once.
+// Measured, whole calls: 1 row 54.4 -> 47.3 us, 64 rows of 32 experts 114.5 -> 104.8, 256 rows (block) 343 -> 338.
+__device__ __forceinline__ void grid_dep_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_sync() {
+  grid_dep_release();
+  grid_dep_wait();
+}
+template <class... Params, class... Args>
+cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, bool chained,
+                          unsigned cluster_y, Args &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  unsigned n = 0;
+  if (chained) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster_y > 0) {   // thread-block clusters of cluster_y CTAs along y
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = 1;
+    at[n].val.clusterDim.y = cluster_y;
+    at[n++].val.clusterDim.z = 1;
+  }
+  cfg.attrs = at;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(std::forward<Args>(args))...);
+}
+
 // What the fused router kernel writes: logits [rows, E], and the selection, weights and expert histogram
 // exactly as topk_softmax_kernel does (to every rank's top-k buffers when tp > 0, at row_offset).
 struct RouteOut {
@@ -271,37 +312,37 @@ struct RouteOut {
 cudaError_t router_init(int *max_cluster);   // per-device kernel attributes; call with the device current
 int router_fused_slices(int T, int H, int E, int sm_count, int max_cluster);
 bool launch_router_fused(const __nv_bfloat16 *t, const CUtensorMap &tm_w, int T, int H, int E, int slices,
-                         const RouteOut &ro, unsigned int *status, cudaStream_t s);
+                         const RouteOut &ro, unsigned int *status, cudaStream_t s, bool chained);
 int router_splits(int T, int H, int sm_count);
 int router_chunks(int H);
 bool make_router_weight_map(CUtensorMap *m, const __nv_bfloat16 *w3, int E, int H);
 bool launch_router_partials(const __nv_bfloat16 *t, const CUtensorMap &tm_w, float *partial, int T, int H, int E,
-                            int splits, unsigned int *status, cudaStream_t s);
+                            int splits, unsigned int *status, cudaStream_t s, bool chained = false);
 // route.cu
 void launch_topk_softmax(float *logits, const float *partial, int splits, const float *bias, int T, int E, int K,
                          int *idx, float *w, int *counts, cudaStream_t s, int tp = 0, const TpPeers *peers = nullptr,
-                         int row_offset = 0);
+                         int row_offset = 0, bool chained = false);
 void launch_count_experts(const int *idx, int n, int E, int *counts, cudaStream_t s);
-void launch_build_index(const int *topk_idx, const int *counts, int T, int E, int K, int n_ntiles1, int n_ntiles2,
+void launch_build_index(const int *topk_idx, const int *hist, int *counts, int T, int E, int K, int n_ntiles1, int n_ntiles2,
                         int *offsets, int *tile_base, int *pair_row, int *row_token, int2 *pair_slot, unsigned int *tile_done, int tile_done_total_slot, WorkItem *work1,
                         WorkItem *work2, int *n_work, int max_work1, int max_work2, unsigned int *status,
-                        cudaStream_t s);
+                        cudaStream_t s, bool chained);
 void launch_quantize_rows(const __nv_bfloat16 *t, const int2 *pair_slot, int T, int K, uint8_t *xq, uint8_t *sfb, int H,
-                          cudaStream_t s);
+                          cudaStream_t s, bool chained);
 int quantize_rows_max_hidden();
 void launch_gather_rows(const __nv_bfloat16 *t, const int *row_token, const int *offsets, int E, __half *xperm,
                         int H, int max_pairs, cudaStream_t s);
 void launch_combine(const __half *y, const int *topk_idx, const float *topk_w, const int *pair_row, int T, int H,
-                    int K, __nv_bfloat16 *out_bf16, float *out_f32, cudaStream_t s, int tp = 0,
+                    int K, __nv_bfloat16 *out_bf16, float *out_f32, int *hist, int E, cudaStream_t s, bool chained, int tp = 0,
                     const TpPeers *peers = nullptr, int rows_local = 0, int rank = 0,
                     const __nv_bfloat16 *residual = nullptr);
 void launch_rmsnorm_rows(const __nv_bfloat16 *x, const __nv_bfloat16 *w, __nv_bfloat16 *t, int rows, int H,
-                         cudaStream_t s);
+                         cudaStream_t s, bool chained);
 
 // expert_gemm_sm100.cu
 cudaError_t expert_gemm_init(int *grid);   // per-device kernel attributes; call with the device current
 void launch_expert_mlp(const CUtensorMap (&tm_w1)[2], const GemmArgs &a, const CUtensorMap (&tm_w2)[2], const GemmArgs &b,
-                       const MlpFuse &f, int grid, cudaStream_t s);
+                       const MlpFuse &f, int grid, cudaStream_t s, bool chained);
 int expert_mlp_done_per_tile(int n_ntiles1);
 
 // tp_collectives.cu

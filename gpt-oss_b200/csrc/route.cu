@@ -30,6 +30,7 @@ __global__ void topk_softmax_kernel(float *__restrict__ logits, const float *__r
                                     const float *__restrict__ bias, int T, int E, int K, int *__restrict__ idx,
                                     float *__restrict__ w, int *__restrict__ counts, int tp, TpPeers peers,
                                     int row_offset) {
+  grid_dep_sync();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= T) return;
   float *row = logits + static_cast<size_t>(row_offset + warp) * E;
@@ -69,6 +70,7 @@ __global__ void topk_softmax_kernel(float *__restrict__ logits, const float *__r
 __global__ void __launch_bounds__(256) count_experts_kernel(const int *__restrict__ idx, int n, int E,
                                                             int *__restrict__ counts) {
   __shared__ int bins[256];
+  grid_dep_sync();
   for (int i = threadIdx.x; i < E; i += blockDim.x) bins[i] = 0;
   __syncthreads();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -86,13 +88,13 @@ void launch_count_experts(const int *idx, int n, int E, int *counts, cudaStream_
 }
 
 void launch_topk_softmax(float *logits, const float *partial, int splits, const float *bias, int T, int E, int K,
-                         int *idx, float *w, int *counts, cudaStream_t s, int tp, const TpPeers *peers, int row_offset) {
+                         int *idx, float *w, int *counts, cudaStream_t s, int tp, const TpPeers *peers, int row_offset, bool chained) {
   const int threads = 128;
   const int blocks = (T * 32 + threads - 1) / threads;
   TpPeers pv = {};
   if (tp > 0 && peers != nullptr) pv = *peers;
-  topk_softmax_kernel<<<blocks, threads, 0, s>>>(logits, partial, splits, bias, T, E, K, idx, w, counts, tp, pv,
-                                                 row_offset);
+  launch_kernel(topk_softmax_kernel, dim3(blocks), threads, 0, s, chained, 0, logits, partial, splits, bias, T, E, K, idx, w,
+                counts, tp, pv, row_offset);
 }
 
 // ---------------------------------------------------------------------------
@@ -102,7 +104,7 @@ void launch_topk_softmax(float *logits, const float *partial, int splits, const 
 // expert are in ascending token order.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024)
-build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ counts, int T, int E, int K,
+build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ hist, int *__restrict__ counts, int T, int E, int K,
                    int n_ntiles1, int n_ntiles2, int *__restrict__ offsets, int *__restrict__ tile_base,
                    int *__restrict__ pair_row, int *__restrict__ row_token, int2 *__restrict__ pair_slot,
                    unsigned int *__restrict__ tile_done, int tile_done_total_slot, WorkItem *__restrict__ work1,
@@ -110,6 +112,7 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ cou
                    unsigned int *status) {
   __shared__ int s_red[2][32];
   __shared__ int s_warp[32];
+  grid_dep_sync();
   const int e = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_warps = blockDim.x >> 5;   // 8, or 32 for batches whose selections 8 warps cannot hold in registers
 
@@ -137,7 +140,7 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ cou
   // exclusive prefix over experts below e: rows and token tiles (its loads travel with the ones above)
   int my_rows = 0, my_tiles = 0;
   for (int i = tid; i < e; i += blockDim.x) {
-    const int c = counts[i];
+    const int c = hist[i];
     my_rows += c;
     my_tiles += expert_tiles(c);
   }
@@ -156,9 +159,10 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ cou
   __syncthreads();   // the only block-wide barrier: prefix partials and hit counts of all warps
   int off = 0, tiles_before = 0;
   for (int i = 0; i < n_warps; ++i) { off += s_red[0][i]; tiles_before += s_red[1][i]; }
-  const int cnt = counts[e];
+  const int cnt = hist[e];
   const int ntt = expert_tiles(cnt), per_tile = tokens_per_tile(cnt);  // this expert's token tiles
   if (tid == 0) {
+    counts[e] = cnt;
     offsets[e] = off;
     tile_base[e] = tiles_before;
     if (e == E - 1) { offsets[E] = off + cnt; tile_base[E] = tiles_before + ntt; }
@@ -219,13 +223,13 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ cou
   }
 }
 
-void launch_build_index(const int *topk_idx, const int *counts, int T, int E, int K, int n_ntiles1, int n_ntiles2,
+void launch_build_index(const int *topk_idx, const int *hist, int *counts, int T, int E, int K, int n_ntiles1, int n_ntiles2,
                         int *offsets, int *tile_base, int *pair_row, int *row_token, int2 *pair_slot,
                         unsigned int *tile_done, int tile_done_total_slot, WorkItem *work1, WorkItem *work2, int *n_work, int max_work1, int max_work2,
-                        unsigned int *status, cudaStream_t s) {
-  build_index_kernel<<<E, T > 2048 ? 1024 : 256, 0, s>>>(topk_idx, counts, T, E, K, n_ntiles1, n_ntiles2, offsets, tile_base,
-                                       pair_row, row_token, pair_slot, tile_done, tile_done_total_slot, work1, work2, n_work,
-                                                          max_work1, max_work2, status);
+                        unsigned int *status, cudaStream_t s, bool chained) {
+  launch_kernel(build_index_kernel, dim3(E), T > 2048 ? 1024 : 256, 0, s, chained, 0, topk_idx, hist, counts, T, E, K, n_ntiles1,
+                n_ntiles2, offsets, tile_base, pair_row, row_token, pair_slot, tile_done, tile_done_total_slot, work1, work2,
+                n_work, max_work1, max_work2, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -249,6 +253,7 @@ template <int kQrVec>         // 6: rows of up to 3072 elements, 8: up to 4096
 __global__ void __launch_bounds__(kQrWarps * 32)
 quantize_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int2 *__restrict__ pair_slot, int T, int K,
                      uint8_t *__restrict__ xq, uint8_t *__restrict__ sfb, int H) {
+  grid_dep_sync();
   const int lane = threadIdx.x & 31;
   const int tok = blockIdx.x * kQrWarps + (threadIdx.x >> 5);
   if (tok >= T) return;   // whole warps leave: no block-wide barrier below
@@ -336,12 +341,10 @@ quantize_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int2 *__restrict
 int quantize_rows_max_hidden() { return 32 * 8 * 16; }
 
 void launch_quantize_rows(const __nv_bfloat16 *t, const int2 *pair_slot, int T, int K, uint8_t *xq, uint8_t *sfb, int H,
-                          cudaStream_t s) {
+                          cudaStream_t s, bool chained) {
   const int blocks = (T + kQrWarps - 1) / kQrWarps;
-  if (H <= 32 * 6 * 16)
-    quantize_rows_kernel<6><<<blocks, kQrWarps * 32, 0, s>>>(t, pair_slot, T, K, xq, sfb, H);
-  else
-    quantize_rows_kernel<8><<<blocks, kQrWarps * 32, 0, s>>>(t, pair_slot, T, K, xq, sfb, H);
+  launch_kernel(H <= 32 * 6 * 16 ? quantize_rows_kernel<6> : quantize_rows_kernel<8>, dim3(blocks), kQrWarps * 32, 0, s, chained,
+                0, t, pair_slot, T, K, xq, sfb, H);
 }
 
 // ---------------------------------------------------------------------------
@@ -389,11 +392,14 @@ template <int kK>
 __global__ void __launch_bounds__(128)
 combine_kernel(const __half *__restrict__ y, const int *__restrict__ topk_idx, const float *__restrict__ topk_w,
                const int *__restrict__ pair_row, int T, int H, int K, __nv_bfloat16 *__restrict__ out_bf16,
-               float *__restrict__ out_f32, int tp, TpPeers peers, int rows_local, int rank,
+               float *__restrict__ out_f32, int *__restrict__ hist, int E, int tp, TpPeers peers, int rows_local, int rank,
                const __nv_bfloat16 *__restrict__ residual) {
   constexpr int kSlots = kK > 0 ? kK : kMaxTopK;
   if (kK > 0) K = kK;
+  grid_dep_sync();
   int t = blockIdx.x;
+  if (t == 0)   // the last kernel of the call that could need it is done: zero for the next call
+    for (int i = threadIdx.x; i < E; i += blockDim.x) hist[i] = 0;
   // tensor-parallel call: the row's bf16 partial goes straight into slot `rank` of the landing buffer of the
   // rank that owns row t (a peer store over NVLink), which is the send half of the reduce-scatter.  Blocks
   // start with the rows of the next rank and end with this rank's own rows, so that the link is busy from the
@@ -480,12 +486,12 @@ combine_kernel(const __half *__restrict__ y, const int *__restrict__ topk_idx, c
 }
 
 void launch_combine(const __half *y, const int *topk_idx, const float *topk_w, const int *pair_row, int T, int H,
-                    int K, __nv_bfloat16 *out_bf16, float *out_f32, cudaStream_t s, int tp, const TpPeers *peers,
-                    int rows_local, int rank, const __nv_bfloat16 *residual) {
+                    int K, __nv_bfloat16 *out_bf16, float *out_f32, int *hist, int E, cudaStream_t s, bool chained, int tp,
+                    const TpPeers *peers, int rows_local, int rank, const __nv_bfloat16 *residual) {
   TpPeers pv = {};
   if (tp > 0 && peers != nullptr) pv = *peers;
-  auto kernel = K == 4 ? combine_kernel<4> : combine_kernel<0>;
-  kernel<<<T, 128, 0, s>>>(y, topk_idx, topk_w, pair_row, T, H, K, out_bf16, out_f32, tp, pv, rows_local, rank, residual);
+  launch_kernel(K == 4 ? combine_kernel<4> : combine_kernel<0>, dim3(T), 128, 0, s, chained, 0, y, topk_idx, topk_w, pair_row, T, H,
+                K, out_bf16, out_f32, hist, E, tp, pv, rows_local, rank, residual);
 }
 
 // ---------------------------------------------------------------------------
@@ -497,6 +503,7 @@ __global__ void __launch_bounds__(256)
 rmsnorm_rows_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w,
                     __nv_bfloat16 *__restrict__ t, int H) {
   __shared__ double s_part[8];
+  grid_dep_sync();
   const uint4 *src = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(blockIdx.x) * H);
   double ss = 0.0;
   for (int c = threadIdx.x; c < H / 8; c += blockDim.x) {
@@ -534,8 +541,8 @@ rmsnorm_rows_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__
 }
 
 void launch_rmsnorm_rows(const __nv_bfloat16 *x, const __nv_bfloat16 *w, __nv_bfloat16 *t, int rows, int H,
-                         cudaStream_t s) {
-  rmsnorm_rows_kernel<<<rows, 256, 0, s>>>(x, w, t, H);
+                         cudaStream_t s, bool chained) {
+  launch_kernel(rmsnorm_rows_kernel, dim3(rows), 256, 0, s, chained, 0, x, w, t, H);
 }
 
 // ---------------------------------------------------------------------------

@@ -105,9 +105,20 @@ router_kernel(const __grid_constant__ CUtensorMap tm_t, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tm = tmem_base;
 
+  grid_dep_release();
   if (warp == 4) {
-    // ---- producer: one activation box and three weight boxes per chunk
+    // ---- producer: one activation box and three weight boxes per chunk.  The weights of the first chunks are on their
+    // way before the wait for the kernel that writes the activations.
     const uint32_t bytes = kRtTile + 3u * static_cast<uint32_t>(n_mma) * kRtK * 2u;
+    const int early = min(n, kRtStages);
+    if (elect_one())
+      for (int s = 0; s < early; ++s) {
+        mbar_arrive_expect_tx(full_bar(s), bytes);
+        for (int pl = 0; pl < 3; ++pl)
+          tma_load_3d(ring + s * kRtStage + (1 + pl) * kRtTile, &tm_w, (c_begin + s) * kRtK, e0, pl, full_bar(s));
+      }
+    __syncwarp();
+    grid_dep_wait();
     for (int i = 0; i < n; ++i) {
       const int s = i % kRtStages;
       if (i >= kRtStages &&
@@ -116,9 +127,10 @@ router_kernel(const __grid_constant__ CUtensorMap tm_t, const __grid_constant__ 
       if (elect_one()) {
         const uint32_t dst = ring + s * kRtStage;
         const int k = (c_begin + i) * kRtK;
-        mbar_arrive_expect_tx(full_bar(s), bytes);
+        if (i >= early) mbar_arrive_expect_tx(full_bar(s), bytes);
         tma_load_2d(dst, &tm_t, k, tok0, full_bar(s));
-        for (int pl = 0; pl < 3; ++pl) tma_load_3d(dst + (1 + pl) * kRtTile, &tm_w, k, e0, pl, full_bar(s));
+        if (i >= early)
+          for (int pl = 0; pl < 3; ++pl) tma_load_3d(dst + (1 + pl) * kRtTile, &tm_w, k, e0, pl, full_bar(s));
       }
       __syncwarp();
     }
@@ -145,6 +157,7 @@ router_kernel(const __grid_constant__ CUtensorMap tm_t, const __grid_constant__ 
       __syncwarp();
     }
   } else if (warp < 4) {
+    grid_dep_wait();
     // ---- result: warp w owns accumulator lanes 32 w .. 32 w + 31 = tokens tok0 + 32 w + lane
     const bool have = n > 0 && mbar_wait_warp(acc_bar, 0u, abort_flag, status, ST_WAIT_DFULL);
     tc_fence_after();
@@ -187,6 +200,7 @@ router_kernel(const __grid_constant__ CUtensorMap tm_t, const __grid_constant__ 
       }
     }
   }
+  grid_dep_wait();   // nothing is written before (the accumulator alone depends on the activations)
   if constexpr (kFused) {
     // every CTA of the cluster has parked its slice; this CTA finishes its share of the 128 tokens
     cg::cluster_group cluster = cg::this_cluster();
@@ -319,14 +333,13 @@ bool make_rows_map(CUtensorMap *m, const __nv_bfloat16 *t, int T, int H) {
 
 // Split-k partial sums for topk_softmax_kernel.  Returns false when the rows have no tensor map.
 bool launch_router_partials(const __nv_bfloat16 *t, const CUtensorMap &tm_w, float *partial, int T, int H, int E,
-                            int splits, unsigned int *status, cudaStream_t s) {
+                            int splits, unsigned int *status, cudaStream_t s, bool chained) {
   CUtensorMap tm_t;
   if (!make_rows_map(&tm_t, t, T, H)) return false;
   const int n_chunks = router_chunks(H), cps = (n_chunks + splits - 1) / splits;
   dim3 grid((T + kRtTok - 1) / kRtTok, splits, (E + kRtExp - 1) / kRtExp);
-  router_kernel<false><<<grid, kRtThreads, kRtSmem, s>>>(tm_t, tm_w, partial, T, H, E, router_mma_n(E), cps, status,
-                                                          RouteOut{});
-  return true;
+  return launch_kernel(router_kernel<false>, grid, kRtThreads, kRtSmem, s, chained, 0, tm_t, tm_w, partial, T, H, E,
+                       router_mma_n(E), cps, status, RouteOut{}) == cudaSuccess;
 }
 
 // Slices of the fused form: a power of two (the 128 tokens of a tile are dealt out evenly), no more than
@@ -342,24 +355,12 @@ int router_fused_slices(int T, int H, int E, int sm_count, int max_cluster) {
 
 // Router GEMM, bias, top-k, softmax and expert histogram in one launch (E <= 128).
 bool launch_router_fused(const __nv_bfloat16 *t, const CUtensorMap &tm_w, int T, int H, int E, int slices,
-                         const RouteOut &ro, unsigned int *status, cudaStream_t s) {
+                         const RouteOut &ro, unsigned int *status, cudaStream_t s, bool chained) {
   CUtensorMap tm_t;
   if (!make_rows_map(&tm_t, t, T, H)) return false;
   const int n_chunks = router_chunks(H), cps = (n_chunks + slices - 1) / slices;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((T + kRtTok - 1) / kRtTok, slices, 1);
-  cfg.blockDim = dim3(kRtThreads, 1, 1);
-  cfg.dynamicSmemBytes = kRtSmem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 1;
-  at[0].val.clusterDim.y = slices;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, router_kernel<true>, tm_t, tm_w, static_cast<float *>(nullptr), T, H, E,
-                            router_mma_n(E), cps, status, ro) == cudaSuccess;
+  return launch_kernel(router_kernel<true>, dim3((T + kRtTok - 1) / kRtTok, slices, 1), kRtThreads, kRtSmem, s, chained, slices,
+                       tm_t, tm_w, static_cast<float *>(nullptr), T, H, E, router_mma_n(E), cps, status, ro) == cudaSuccess;
 }
 
 }  // namespace moe
