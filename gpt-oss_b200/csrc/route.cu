@@ -103,6 +103,9 @@ void launch_topk_softmax(float *logits, const float *partial, int splits, const 
 // route_build_index_kernel_bf16wts (kernels/moe.hpp:1173-1270): rows of one
 // expert are in ascending token order.
 // ---------------------------------------------------------------------------
+// kK: experts per token known at compile time, 0: any.  The loops are kept rolled: at small batches this kernel, like the
+// quantiser below, takes as long as its instructions take to arrive (each layer's weights push the code out of the caches).
+template <int kK>
 __global__ void __launch_bounds__(1024)
 build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ hist, int *__restrict__ counts, int T, int E, int K,
                    int n_ntiles1, int n_ntiles2, int *__restrict__ offsets, int *__restrict__ tile_base,
@@ -118,27 +121,28 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ his
 
   // Stable compaction in ascending token order.  Warp w owns the contiguous token range [w*per, (w+1)*per):
   // a first walk counts the range's hits with ballots, the block's one barrier turns the warps' counts into
-  // starting positions, a second walk writes the rows.
+  // starting positions, a second walk (its loads hit L1) writes the rows.
   const int per = ((T + n_warps - 1) / n_warps + 31) / 32 * 32;       // tokens per warp, whole ballot steps
   const int t_begin = warp * per, t_end = min(T, t_begin + per);
   auto hit_of = [&](int t) -> int {
     if (t >= t_end) return -1;
-    if (K == 4) {                                      // the usual case: one 16-byte load
+    if constexpr (kK == 4) {                           // the usual case: one 16-byte load
       const int4 v = __ldg(reinterpret_cast<const int4 *>(topk_idx) + t);
       return v.x == e ? 0 : v.y == e ? 1 : v.z == e ? 2 : v.w == e ? 3 : -1;
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < K; ++k)
+        if (__ldg(topk_idx + static_cast<size_t>(t) * K + k) == e) return k;
+      return -1;
     }
-    for (int k = 0; k < K; ++k)
-      if (topk_idx[static_cast<size_t>(t) * K + k] == e) return k;
-    return -1;
   };
-  // the first kCached ballot steps of the range (all of it up to 256 tokens per warp) are loaded at once and kept
-  constexpr int kCached = 8;
-  int cached[kCached];
-#pragma unroll
-  for (int j = 0; j < kCached; ++j) cached[j] = hit_of(t_begin + 32 * j + lane);
+  int mine = 0;
+#pragma unroll 4
+  for (int t0 = t_begin; t0 < t_end; t0 += 32) mine += __popc(__ballot_sync(0xffffffffu, hit_of(t0 + lane) >= 0));
 
   // exclusive prefix over experts below e: rows and token tiles (its loads travel with the ones above)
   int my_rows = 0, my_tiles = 0;
+#pragma unroll 1
   for (int i = tid; i < e; i += blockDim.x) {
     const int c = hist[i];
     my_rows += c;
@@ -149,15 +153,10 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ his
     my_rows += __shfl_xor_sync(0xffffffffu, my_rows, off);
     my_tiles += __shfl_xor_sync(0xffffffffu, my_tiles, off);
   }
-  // first walk: this warp's hits
-  const int t_rest = t_begin + 32 * kCached;
-  int mine = 0;
-#pragma unroll
-  for (int j = 0; j < kCached; ++j) mine += __popc(__ballot_sync(0xffffffffu, cached[j] >= 0));
-  for (int t0 = t_rest; t0 < t_end; t0 += 32) mine += __popc(__ballot_sync(0xffffffffu, hit_of(t0 + lane) >= 0));
   if (lane == 0) { s_red[0][warp] = my_rows; s_red[1][warp] = my_tiles; s_warp[warp] = mine; }
   __syncthreads();   // the only block-wide barrier: prefix partials and hit counts of all warps
   int off = 0, tiles_before = 0;
+#pragma unroll 4
   for (int i = 0; i < n_warps; ++i) { off += s_red[0][i]; tiles_before += s_red[1][i]; }
   const int cnt = hist[e];
   const int ntt = expert_tiles(cnt), per_tile = tokens_per_tile(cnt);  // this expert's token tiles
@@ -168,10 +167,12 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ his
     if (e == E - 1) { offsets[E] = off + cnt; tile_base[E] = tiles_before + ntt; }
   }
   // completion counters of the fused expert MLP launch: this expert's token tiles, and the total
+#pragma unroll 1
   for (int i = tid; i < ntt; i += blockDim.x) tile_done[tiles_before + i] = 0u;
   if (e == E - 1 && tid == 0) tile_done[tile_done_total_slot] = 0u;
 
   int before = 0, total_hits = 0;
+#pragma unroll 4
   for (int i = 0; i < n_warps; ++i) {
     before += i < warp ? s_warp[i] : 0;
     total_hits += s_warp[i];
@@ -194,18 +195,19 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ his
     }
     before += __popc(m);
   };
-#pragma unroll
-  for (int j = 0; j < kCached; ++j) place(t_begin + 32 * j + lane, cached[j]);
-  for (int t0 = t_rest; t0 < t_end; t0 += 32) place(t0 + lane, hit_of(t0 + lane));
+#pragma unroll 1
+  for (int t0 = t_begin; t0 < t_end; t0 += 32) place(t0 + lane, hit_of(t0 + lane));
   if (tid == 0 && total_hits != cnt) atomicOr(status, ST_BAD_INDEX);
 
   // work items: one per (token tile, block of kBlockRows weight rows); items that share a
   // weight block are adjacent so that block is fetched from HBM once and re-read from L2.
+#pragma unroll 1
   for (int which = 0; which < 2; ++which) {
     const int nn = which ? n_ntiles2 : n_ntiles1;
     WorkItem *work = which ? work2 : work1;
     const int cap = which ? max_work2 : max_work1;
     const int start = tiles_before * nn;
+#pragma unroll 1
     for (int i = tid; i < ntt * nn; i += blockDim.x) {
       const int nt = i / ntt, tt = i % ntt;
       WorkItem it;
@@ -227,7 +229,7 @@ void launch_build_index(const int *topk_idx, const int *hist, int *counts, int T
                         int *offsets, int *tile_base, int *pair_row, int *row_token, int2 *pair_slot,
                         unsigned int *tile_done, int tile_done_total_slot, WorkItem *work1, WorkItem *work2, int *n_work, int max_work1, int max_work2,
                         unsigned int *status, cudaStream_t s, bool chained) {
-  launch_kernel(build_index_kernel, dim3(E), T > 2048 ? 1024 : 256, 0, s, chained, 0, topk_idx, hist, counts, T, E, K, n_ntiles1,
+  launch_kernel(K == 4 ? build_index_kernel<4> : build_index_kernel<0>, dim3(E), T > 2048 ? 1024 : 256, 0, s, chained, 0, topk_idx, hist, counts, T, E, K, n_ntiles1,
                 n_ntiles2, offsets, tile_base, pair_row, row_token, pair_slot, tile_done, tile_done_total_slot, work1, work2,
                 n_work, max_work1, max_work2, status);
 }
@@ -244,10 +246,16 @@ void launch_build_index(const int *topk_idx, const int *hist, int *counts, int T
 // (127+e, 127+e-4) go into the tile's 512-byte scale atoms, byte (r%32)*16 + (r/32 %4)*4 + kb of atom r/128 for
 // operand row r and every k block kb (the scale is per row, so the four bytes are equal).
 // ---------------------------------------------------------------------------
-// The two rows depend on the token only, not on the expert, so a warp quantises one TOKEN (its row stays in
-// the warp's registers: kQrVec x 32 bytes per lane) and stores the result once per selected expert, at the
-// tile rows build_index_kernel assigned to the (token, expert) pairs.
+// The two rows depend on the token only, not on the expert, so a warp quantises one TOKEN and stores the result once per
+// selected expert, at the tile rows build_index_kernel assigned to the (token, expert) pairs.  Two forms:
+//  * up to kQrFewRows rows: rolled loops, two passes over the row (the second out of L1), 9 KB of code.  A small batch
+//    waits for the code to be fetched (each layer's weights push it out of the caches), and that is most of the kernel's
+//    time: with the 52 KB of the other form, and an index kernel twice the size, a call with 1 row took 45.2 us instead of
+//    39.3, 32 rows 186.7 / 184.5, 256 rows (block) 331 / 327.
+//  * larger batches: the row stays in registers (kQrVec x 32 bytes per lane), bound by the writes; the rolled form takes
+//    46 us instead of 41 at 7424 rows, and the same at 1536.
 constexpr int kQrWarps = 4;
+constexpr int kQrFewRows = 512;
 
 template <int kQrVec>         // 6: rows of up to 3072 elements, 8: up to 4096
 __global__ void __launch_bounds__(kQrWarps * 32)
@@ -338,12 +346,90 @@ quantize_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int2 *__restrict
   }
 }
 
+template <int kK>             // experts per token known at compile time, 0: any up to kMaxTopK
+__global__ void __launch_bounds__(kQrWarps * 32)
+quantize_few_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int2 *__restrict__ pair_slot, int T, int K,
+                     uint8_t *__restrict__ xq, uint8_t *__restrict__ sfb, int H) {
+  constexpr int kSlots = kK > 0 ? kK : kMaxTopK;
+  if (kK > 0) K = kK;
+  grid_dep_sync();
+  const int lane = threadIdx.x & 31;
+  const int tok = blockIdx.x * kQrWarps + (threadIdx.x >> 5);
+  if (tok >= T) return;   // whole warps leave: no block-wide barrier below
+  int2 slot[kSlots];
+#pragma unroll
+  for (int k = 0; k < kSlots; ++k) slot[k] = k < K ? pair_slot[static_cast<size_t>(tok) * K + k] : make_int2(-1, 0);
+  const uint4 *src = reinterpret_cast<const uint4 *>(t + static_cast<size_t>(tok) * H);
+  const int ngrp = H / 16;    // a lane takes groups of 16 elements: 32 bytes in, 16 + 16 bytes out
+  // Largest magnitude: bf16 magnitudes compare like their bit patterns.  (A NaN wins, and every output of its token is
+  // NaN whatever the scale.)
+  uint32_t top = 0;
+#pragma unroll 6
+  for (int g = lane; g < ngrp; g += 32) {
+    const uint4 a = __ldg(src + 2 * g), b = __ldg(src + 2 * g + 1);
+    const uint32_t in[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) top = __vmaxu2(top, in[j] & 0x7fff7fffu);
+  }
+#pragma unroll
+  for (int off = 16; off; off >>= 1) top = __vmaxu2(top, __shfl_xor_sync(0xffffffffu, top, off));
+  top = max(top & 0xffffu, top >> 16);
+  // e = floor(log2(amax)) - 7, kept where both scales stay valid UE8M0 bytes
+  int e = static_cast<int>(top >> 7) - 127 - 7;
+  e = max(-120, min(e, 120));
+  const float inv = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);  // 2^-e
+  // activation tiles: see x_pair_offset; 16 elements never straddle a slice
+  const int n_pairs = slice_pairs((H + kChunkK - 1) / kChunkK);
+#pragma unroll 1
+  for (int g = lane; g < ngrp; g += 32) {
+    uint32_t h8[4], l8[4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint4 v = __ldg(src + 2 * g + h);
+      const uint32_t in[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        uint32_t hi[2], lo[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float f0 = __uint_as_float(in[2 * q + j] << 16) * inv, f1 = __uint_as_float(in[2 * q + j] & 0xffff0000u) * inv;
+          hi[j] = __nv_cvt_float2_to_fp8x2(make_float2(f0, f1), __NV_SATFINITE, __NV_E4M3);
+          const float2 back = __half22float2(__half2(__nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(hi[j]), __NV_E4M3)));
+          lo[j] = __nv_cvt_float2_to_fp8x2(make_float2((f0 - back.x) * 16.0f, (f1 - back.y) * 16.0f), __NV_SATFINITE, __NV_E4M3);
+        }
+        h8[2 * h + q] = hi[0] | (hi[1] << 16);
+        l8[2 * h + q] = lo[0] | (lo[1] << 16);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kSlots; ++k) {
+      if (slot[k].x < 0) continue;
+      const int tile = slot[k].x / kMaxTileTok, i = slot[k].x % kMaxTileTok;
+      uint8_t *dst = xq + (static_cast<size_t>(tile) * n_pairs + (g >> 4)) * kPairBytes;   // 16 groups to a pair of slices
+      *reinterpret_cast<uint4 *>(dst + x_pair_offset(i, 0, (g & 15) * 16)) = make_uint4(h8[0], h8[1], h8[2], h8[3]);
+      *reinterpret_cast<uint4 *>(dst + x_pair_offset(i, 1, (g & 15) * 16)) = make_uint4(l8[0], l8[1], l8[2], l8[3]);
+    }
+  }
+  if (lane < 2) {
+    const uint32_t byte = static_cast<uint32_t>(127 + e - 4 * lane);
+#pragma unroll
+    for (int k = 0; k < kSlots; ++k) {
+      if (slot[k].x < 0) continue;
+      const int tile = slot[k].x / kMaxTileTok, rr = slot[k].y + lane;  // operand row: even = high, odd = low
+      uint8_t *atom = sfb + static_cast<size_t>(tile) * kSfbTileBytes + rr / 128 * kSfAtomBytes;
+      *reinterpret_cast<uint32_t *>(atom + (rr % 32) * 16 + (rr / 32 % 4) * 4) = byte * 0x01010101u;
+    }
+  }
+}
+
 int quantize_rows_max_hidden() { return 32 * 8 * 16; }
 
 void launch_quantize_rows(const __nv_bfloat16 *t, const int2 *pair_slot, int T, int K, uint8_t *xq, uint8_t *sfb, int H,
                           cudaStream_t s, bool chained) {
   const int blocks = (T + kQrWarps - 1) / kQrWarps;
-  launch_kernel(H <= 32 * 6 * 16 ? quantize_rows_kernel<6> : quantize_rows_kernel<8>, dim3(blocks), kQrWarps * 32, 0, s, chained,
+  auto kernel = T <= kQrFewRows ? (K == 4 ? quantize_few_rows_kernel<4> : quantize_few_rows_kernel<0>)
+                                : (H <= 32 * 6 * 16 ? quantize_rows_kernel<6> : quantize_rows_kernel<8>);
+  launch_kernel(kernel, dim3(blocks), kQrWarps * 32, 0, s, chained,
                 0, t, pair_slot, T, K, xq, sfb, H);
 }
 
