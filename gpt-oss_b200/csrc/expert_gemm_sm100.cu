@@ -40,11 +40,11 @@
 // One more warp counts finished MLP1 items for the MLP2 items that wait for them.
 // No multicast: every CTA fetches its own tiles.
 //
-// Measured (B200, one launch of both phases, us, layer of 128 experts, hidden and
-// intermediate size 2880; before: one CTA per item of 64 tokens x 240 rows, tokens on the fixed M = 128 axis): 32 rows 179 -> 174,
-// 256 rows 324 -> 299, 1856 rows 412 -> 396, 8192 rows 1459 -> 1403.  Alone at 256 rows the copies take 269 (HBM at its
-// peak) and the MMAs 214: what is left is the round trip of the ring.  At 8192 rows the tensor pipe is busy 87 % of
-// the cycles and the power cap sets the clock (1.29 GHz).
+// Measured (B200, one launch of both phases, us, layer of 128 experts, hidden and intermediate size 2880; before: one CTA
+// per item of 64 tokens x 240 rows, tokens on the fixed M = 128 axis), without the L2 prefetch further down: 32 rows
+// 179 -> 174, 256 rows 324 -> 299, 1856 rows 412 -> 396, 8192 rows 1459 -> 1403.  Bound by HBM up to ~16 tokens per
+// expert, by the shared-memory port around 60 (712 of 773 cycles per stage), by the tensor pipe above (86 % of the cycles
+// at 8192 rows, where the power cap sets the clock to 1.29 GHz).
 #include <cuda_fp8.h>
 
 #include "moe_internal.cuh"
