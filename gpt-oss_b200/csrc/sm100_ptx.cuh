@@ -35,9 +35,6 @@ __device__ __forceinline__ void fence_mbar_init() {
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
@@ -72,27 +69,11 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait.  `abort_flag` is a CTA-shared word that any role sets when it
+// Bounded wait of a whole converged warp.  `abort_flag` is a CTA-shared word that any role sets when it
 // gives up; `status` is the global status word the host reads.  About one
 // second of polling at most, and it leaves early once another role aborted.
 constexpr long long kWaitCycles = 2000000000LL;
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag,
-                                          unsigned int *status, unsigned int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  for (uint32_t spin = 0;; ++spin) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((spin & 63u) == 63u) {
-      if (*abort_flag) return false;
-      if (clock64() - t0 > kWaitCycles) break;
-    }
-  }
-  *abort_flag = 1u;
-  atomicOr(status, code);
-  return false;
-}
-
-// The same wait for a whole converged warp.  Every decision is taken by a vote, so the 32 lanes leave
+// Every decision is taken by a vote, so the 32 lanes leave
 // together (success or give-up) and may go on to warp-wide instructions (elect.sync).  The roles that
 // issue tcgen05.mma or TMA keep their warp converged and elect one lane per instruction group: the
 // operands of those instructions (descriptors, tensor-memory addresses) are then computed once per warp in
