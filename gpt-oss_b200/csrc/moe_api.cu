@@ -109,6 +109,21 @@ void tile_weights(const uint8_t *codes, size_t pitch, size_t row_bytes, const ui
     }
 }
 
+// The expert histogram is zero between calls: the combine kernel clears it behind the last kernel that reads it.  A call
+// that fails after something may have counted into it clears it here, in the order of its own stream, so that whatever
+// runs on the handle next finds zeros: the next call, a graph captured before this one, or, when this call is itself being
+// captured, the rest of that graph.  (No flag on the host could say so: a captured call runs later, or never.)
+struct HistogramGuard {
+  int *hist;
+  int n;
+  cudaStream_t stream;
+  bool armed = false;
+  ~HistogramGuard() {
+    if (armed && cudaMemsetAsync(hist, 0, sizeof(int) * n, stream) != cudaSuccess)
+      (void)cudaGetLastError();   // the stream takes no more work: nothing was launched on it either
+  }
+};
+
 void free_layer(LayerWeights &w) {
   cudaFree(w.w1_tiles); cudaFree(w.b1);
   cudaFree(w.w2_tiles); cudaFree(w.b2);
@@ -139,8 +154,7 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
   // The kernels of a one-GPU call are chained by programmatic dependent launch; a profile's events between them, and the
   // side stream and hand-shakes of a group's call, want ordinary launches.
   const bool chained = !tpcall && !c->profiling;
-  if (c->hist_dirty) CU_TRY(c, cudaMemsetAsync(c->hist, 0, sizeof(int) * E, s));
-  c->hist_dirty = true;
+  HistogramGuard guard{c->hist, E, s};
   auto mark = [&]() {
     if (!c->profiling) return;
     cudaEvent_t ev;
@@ -171,6 +185,7 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
     if (tpcall) { ro.tp = tp; ro.peers = c->peers; ro.row_offset = rank * tp_rows_local; }
     else { ro.idx = c->topk_idx; ro.w = c->topk_w; ro.counts = c->hist; }
     bool ok;
+    guard.armed = !tpcall;   // the routing kernels count (in a TP call launch_count_experts does)
     if (slices > 0) {
       ok = launch_router_fused(src, w.tm_router, n, H, E, slices, ro, status, s, chained);
       routed_in_one_launch = true;
@@ -180,8 +195,8 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
       const int splits = router_splits(n, H, c->sm_count);
       ok = launch_router_partials(src, w.tm_router, c->router_part, n, H, E, splits, status, s, chained);
       mark();
-      launch_topk_softmax(ro.logits, c->router_part, splits, ro.bias, n, E, K, ro.idx, ro.w, ro.counts, s, ro.tp,
-                          &ro.peers, ro.row_offset, chained);
+      if (ok) launch_topk_softmax(ro.logits, c->router_part, splits, ro.bias, n, E, K, ro.idx, ro.w, ro.counts, s, ro.tp,
+                                  &ro.peers, ro.row_offset, chained);
     }
     if (!ok) return fail(c, MOE_ERR_INVALID, "router launch refused (input rows 16-byte aligned, hidden_dim a multiple of 8?)");
     return MOE_OK;
@@ -216,6 +231,7 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
       c->launches += 1;
     }
     CU_TRY(c, cudaEventRecord(c->ev_join, c->aux_stream));
+    guard.armed = true;
     launch_count_experts(c->topk_idx, T * K, E, c->hist, s);
     mark();
     c->launches += 4;
@@ -289,7 +305,7 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
   c->launches += 7;
   c->last_rows = rows;
   CU_TRY(c, cudaGetLastError());
-  c->hist_dirty = false;
+  guard.armed = false;
   return MOE_OK;
 }
 

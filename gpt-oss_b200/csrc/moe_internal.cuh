@@ -194,8 +194,8 @@ struct moe_ctx {
   float *router_part = nullptr;     // split-k partial sums of the router [splits, rows, E]
   int *topk_idx = nullptr;          // topk_i_g            [max_rows, K]
   float *topk_w = nullptr;          // topk_v_g            [max_rows, K]
-  int *hist = nullptr;              // selections per expert of the running call [E]; zero between calls (combine clears it)
-  bool hist_dirty = false;          // a call did not get as far as clearing it
+  int *hist = nullptr;              // selections per expert of the running call [E]; zero between calls (combine clears it,
+                                    // or the failing call itself)
   int *counts = nullptr;            // d_expert_counts     [E]   hist of the last call, kept
   int *offsets = nullptr;           // d_expert_offsets    [E+1]
   int *pair_row = nullptr;          // local_ids_g         [max_rows, K]

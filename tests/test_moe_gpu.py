@@ -531,6 +531,61 @@ def test_forward_in_a_cuda_graph(pkg, synth):
         blk.close()
 
 
+@pytest.mark.parametrize("E,flags", [(16, 0), (16, 4), (160, 0)], ids=["fused", "split_router", "160_experts"])
+def test_a_refused_call_leaves_graphs_and_later_calls_alone(E, flags, pkg, synth):
+    """Rows that the router refuses (not 16-byte aligned) are an error and nothing else: a graph captured before, one
+    captured after it, and eager calls before that graph's first replay give the bits of a call on a fresh handle."""
+    import torch
+    H, D, T = 128, 64, 40
+    layer, rows = synth.make_layer(E, H, D, seed=61), synth.make_tokens(T, H, seed=62)
+    blk = pkg.MoeBlock(H, D, E, max_rows=4 * T)
+    try:
+        blk.load_layer(0, layer)
+        want = blk.forward_host(0, rows, flags=flags).copy()
+        d_t = torch.zeros(T * H + 8, dtype=torch.int16, device="cuda")
+        d_t[:T * H] = torch.from_numpy(rows.view(np.int16)).cuda().reshape(-1)
+        d_o = torch.zeros((T, H), dtype=torch.int16, device="cuda")
+        s = torch.cuda.Stream()
+
+        def call(ptr):
+            blk.forward(0, ptr, T, d_o.data_ptr(), flags, torch.cuda.current_stream().cuda_stream)
+
+        def refused():
+            with pytest.raises(pkg.MoeError) as ei:
+                call(d_t.data_ptr() + 2)
+            assert ei.value.code == 1
+
+        def check(run):
+            d_o.zero_()
+            run()
+            torch.cuda.synchronize()
+            blk.synchronize()
+            assert np.array_equal(d_o.cpu().numpy().view(np.uint16), want)
+
+        torch.cuda.synchronize()
+        with torch.cuda.stream(s):
+            check(lambda: call(d_t.data_ptr()))
+            before, after, within = (torch.cuda.CUDAGraph() for _ in range(3))
+            with torch.cuda.graph(before, stream=s):
+                call(d_t.data_ptr())
+            check(before.replay)
+            refused()
+            check(before.replay)             # captured before the refused call
+            refused()
+            with torch.cuda.graph(after, stream=s):
+                call(d_t.data_ptr())
+            check(lambda: call(d_t.data_ptr()))   # nothing of the second graph has run yet
+            check(after.replay)
+            with torch.cuda.graph(within, stream=s):
+                refused()
+                call(d_t.data_ptr())
+            for _ in range(2):
+                check(within.replay)
+                check(lambda: call(d_t.data_ptr()))
+    finally:
+        blk.close()
+
+
 def test_expert_output_beyond_fp16_is_reported(pkg, synth):
     """The per-(token, expert) MLP2 outputs wait for the combine in fp16; a magnitude above 65504 is an
     error code, not a silent infinity, and the handle keeps working."""
