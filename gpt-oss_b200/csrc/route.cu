@@ -26,10 +26,8 @@ namespace moe {
 // With tp > 0 the call routes rows [row_offset, row_offset + T) of a tensor-parallel group's union batch:
 // logits go to those rows of `logits`, and the selection is written into the top-k buffers of every rank
 // of the group (peer stores), so that no rank repeats another rank's routing.
-__global__ void topk_softmax_kernel(float *__restrict__ logits, const float *__restrict__ partial, int splits,
-                                    const float *__restrict__ bias, int T, int E, int K, int *__restrict__ idx,
-                                    float *__restrict__ w, int *__restrict__ counts, int tp, TpPeers peers,
-                                    int row_offset) {
+__global__ void topk_softmax_kernel(float *logits, const float *partial, int splits, const float *__restrict__ bias, int T,
+                                    int E, int K, int *idx, float *w, int *counts, int tp, TpPeers peers, int row_offset) {
   grid_dep_sync();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= T) return;
@@ -67,8 +65,7 @@ __global__ void topk_softmax_kernel(float *__restrict__ logits, const float *__r
 
 // Expert histogram over an already exchanged selection (count_tokens_per_expert_kernel,
 // kernels/moe.hpp:744); block-local bins first, so global atomics are E per block.
-__global__ void __launch_bounds__(256) count_experts_kernel(const int *__restrict__ idx, int n, int E,
-                                                            int *__restrict__ counts) {
+__global__ void __launch_bounds__(256) count_experts_kernel(const int *idx, int n, int E, int *counts) {
   __shared__ int bins[256];
   grid_dep_sync();
   for (int i = threadIdx.x; i < E; i += blockDim.x) bins[i] = 0;
@@ -107,11 +104,9 @@ void launch_topk_softmax(float *logits, const float *partial, int splits, const 
 // quantiser below, takes as long as its instructions take to arrive (each layer's weights push the code out of the caches).
 template <int kK>
 __global__ void __launch_bounds__(1024)
-build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ hist, int *__restrict__ counts, int T, int E, int K,
-                   int n_ntiles1, int n_ntiles2, int *__restrict__ offsets, int *__restrict__ tile_base,
-                   int *__restrict__ pair_row, int *__restrict__ row_token, int2 *__restrict__ pair_slot,
-                   unsigned int *__restrict__ tile_done, int tile_done_total_slot, WorkItem *__restrict__ work1,
-                   WorkItem *__restrict__ work2, int *__restrict__ n_work, int max_work1, int max_work2,
+build_index_kernel(const int *topk_idx, const int *hist, int *counts, int T, int E, int K, int n_ntiles1, int n_ntiles2,
+                   int *offsets, int *tile_base, int *pair_row, int *row_token, int2 *pair_slot, unsigned int *tile_done,
+                   int tile_done_total_slot, WorkItem *work1, WorkItem *work2, int *n_work, int max_work1, int max_work2,
                    unsigned int *status) {
   __shared__ int s_red[2][32];
   __shared__ int s_warp[32];
@@ -127,12 +122,12 @@ build_index_kernel(const int *__restrict__ topk_idx, const int *__restrict__ his
   auto hit_of = [&](int t) -> int {
     if (t >= t_end) return -1;
     if constexpr (kK == 4) {                           // the usual case: one 16-byte load
-      const int4 v = __ldg(reinterpret_cast<const int4 *>(topk_idx) + t);
+      const int4 v = reinterpret_cast<const int4 *>(topk_idx)[t];
       return v.x == e ? 0 : v.y == e ? 1 : v.z == e ? 2 : v.w == e ? 3 : -1;
     } else {
 #pragma unroll 1
       for (int k = 0; k < K; ++k)
-        if (__ldg(topk_idx + static_cast<size_t>(t) * K + k) == e) return k;
+        if (topk_idx[static_cast<size_t>(t) * K + k] == e) return k;
       return -1;
     }
   };
@@ -259,8 +254,7 @@ constexpr int kQrFewRows = 512;
 
 template <int kQrVec>         // 6: rows of up to 3072 elements, 8: up to 4096
 __global__ void __launch_bounds__(kQrWarps * 32)
-quantize_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int2 *__restrict__ pair_slot, int T, int K,
-                     uint8_t *__restrict__ xq, uint8_t *__restrict__ sfb, int H) {
+quantize_rows_kernel(const __nv_bfloat16 *t, const int2 *pair_slot, int T, int K, uint8_t *xq, uint8_t *sfb, int H) {
   grid_dep_sync();
   const int lane = threadIdx.x & 31;
   const int tok = blockIdx.x * kQrWarps + (threadIdx.x >> 5);
@@ -277,7 +271,7 @@ quantize_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int2 *__restrict
     const int g = lane + u * 32;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      v[u][h] = g < ngrp ? __ldg(src + 2 * g + h) : make_uint4(0u, 0u, 0u, 0u);
+      v[u][h] = g < ngrp ? src[2 * g + h] : make_uint4(0u, 0u, 0u, 0u);
       const uint32_t in[4] = {v[u][h].x, v[u][h].y, v[u][h].z, v[u][h].w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -348,8 +342,7 @@ quantize_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int2 *__restrict
 
 template <int kK>             // experts per token known at compile time, 0: any up to kMaxTopK
 __global__ void __launch_bounds__(kQrWarps * 32)
-quantize_few_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int2 *__restrict__ pair_slot, int T, int K,
-                     uint8_t *__restrict__ xq, uint8_t *__restrict__ sfb, int H) {
+quantize_few_rows_kernel(const __nv_bfloat16 *t, const int2 *pair_slot, int T, int K, uint8_t *xq, uint8_t *sfb, int H) {
   constexpr int kSlots = kK > 0 ? kK : kMaxTopK;
   if (kK > 0) K = kK;
   grid_dep_sync();
@@ -366,7 +359,7 @@ quantize_few_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int2 *__rest
   uint32_t top = 0;
 #pragma unroll 6
   for (int g = lane; g < ngrp; g += 32) {
-    const uint4 a = __ldg(src + 2 * g), b = __ldg(src + 2 * g + 1);
+    const uint4 a = src[2 * g], b = src[2 * g + 1];
     const uint32_t in[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
     for (int j = 0; j < 8; ++j) top = __vmaxu2(top, in[j] & 0x7fff7fffu);
@@ -385,7 +378,7 @@ quantize_few_rows_kernel(const __nv_bfloat16 *__restrict__ t, const int2 *__rest
     uint32_t h8[4], l8[4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const uint4 v = __ldg(src + 2 * g + h);
+      const uint4 v = src[2 * g + h];
       const uint32_t in[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
@@ -476,10 +469,9 @@ void launch_gather_rows(const __nv_bfloat16 *t, const int *row_token, const int 
 // one is finished.  kK: experts per token known at compile time, 0: any K up to kMaxTopK (predicated).
 template <int kK>
 __global__ void __launch_bounds__(128)
-combine_kernel(const __half *__restrict__ y, const int *__restrict__ topk_idx, const float *__restrict__ topk_w,
-               const int *__restrict__ pair_row, int T, int H, int K, __nv_bfloat16 *__restrict__ out_bf16,
-               float *__restrict__ out_f32, int *__restrict__ hist, int E, int tp, TpPeers peers, int rows_local, int rank,
-               const __nv_bfloat16 *__restrict__ residual) {
+combine_kernel(const __half *y, const int *topk_idx, const float *topk_w, const int *pair_row, int T, int H, int K,
+               __nv_bfloat16 *out_bf16, float *out_f32, int *hist, int E, int tp, TpPeers peers, int rows_local, int rank,
+               const __nv_bfloat16 *residual) {
   constexpr int kSlots = kK > 0 ? kK : kMaxTopK;
   if (kK > 0) K = kK;
   grid_dep_sync();
@@ -525,7 +517,7 @@ combine_kernel(const __half *__restrict__ y, const int *__restrict__ topk_idx, c
   auto fetch = [&](int i) {
 #pragma unroll
     for (int k = 0; k < kSlots; ++k)
-      if (k < K && i < n_vec) raw[k] = __ldg(src[k] + i);
+      if (k < K && i < n_vec) raw[k] = src[k][i];
   };
   fetch(threadIdx.x);
   for (int i = threadIdx.x; i < n_vec; i += blockDim.x) {
@@ -551,7 +543,7 @@ combine_kernel(const __half *__restrict__ y, const int *__restrict__ topk_idx, c
       o[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
     }
     if (residual != nullptr) {  // x += block output (accumulate_kernel_bf16, kernels/other_kernels.hpp:18-37), one rounding
-      const uint4 r = __ldg(reinterpret_cast<const uint4 *>(residual + static_cast<size_t>(t) * H) + i);
+      const uint4 r = reinterpret_cast<const uint4 *>(residual + static_cast<size_t>(t) * H)[i];
       const uint32_t r4[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -586,14 +578,13 @@ void launch_combine(const __half *y, const int *topk_idx, const float *topk_w, c
 // and rmsnorm of the CPU path (run.cpp:320-333).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-rmsnorm_rows_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w,
-                    __nv_bfloat16 *__restrict__ t, int H) {
+rmsnorm_rows_kernel(const __nv_bfloat16 *x, const __nv_bfloat16 *w, __nv_bfloat16 *t, int H) {
   __shared__ double s_part[8];
   grid_dep_sync();
   const uint4 *src = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(blockIdx.x) * H);
   double ss = 0.0;
   for (int c = threadIdx.x; c < H / 8; c += blockDim.x) {
-    const uint4 v = __ldg(src + c);
+    const uint4 v = src[c];
     const uint32_t in[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -612,7 +603,7 @@ rmsnorm_rows_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__
   const uint4 *wv = reinterpret_cast<const uint4 *>(w);
   uint4 *dst = reinterpret_cast<uint4 *>(t + static_cast<size_t>(blockIdx.x) * H);
   for (int c = threadIdx.x; c < H / 8; c += blockDim.x) {
-    const uint4 v = __ldg(src + c), g = __ldg(wv + c);
+    const uint4 v = src[c], g = wv[c];
     const uint32_t in[4] = {v.x, v.y, v.z, v.w}, gn[4] = {g.x, g.y, g.z, g.w};
     uint32_t o[4];
 #pragma unroll

@@ -19,8 +19,8 @@ constexpr int kMaxTopK = 8;
 // rank of a tensor-parallel group when tp > 0) and adds the selection to the expert histogram.
 template <bool kContig = false>
 __device__ __forceinline__ void select_softmax_store(const float (&v)[kMaxExpPerLane], unsigned taken, int lane, int K,
-                                                     size_t out_row, int *__restrict__ idx, float *__restrict__ w,
-                                                     int *__restrict__ counts, int tp, const TpPeers &peers) {
+                                                     size_t out_row, int *idx, float *w, int *counts, int tp,
+                                                     const TpPeers &peers) {
   float sel_v = 0.f;  // lane k keeps the k-th selected logit
   int sel_i = 0;
   for (int k = 0; k < K; ++k) {

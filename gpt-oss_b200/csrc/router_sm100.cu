@@ -65,7 +65,7 @@ __device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uin
 template <bool kFused>
 __global__ void __launch_bounds__(kRtThreads, 1)
 router_kernel(const __grid_constant__ CUtensorMap tm_t, const __grid_constant__ CUtensorMap tm_w,
-              float *__restrict__ partial, int T, int H, int E, int n_mma, int chunks_per_split,
+              float *partial, int T, int H, int E, int n_mma, int chunks_per_split,
               unsigned int *status, RouteOut ro) {
   extern __shared__ uint8_t rt_raw[];
   const uint32_t ring = (smem_u32(rt_raw) + 1023u) & ~1023u;

@@ -586,6 +586,67 @@ def test_a_refused_call_leaves_graphs_and_later_calls_alone(E, flags, pkg, synth
         blk.close()
 
 
+def test_calls_directly_behind_one_another(pkg, synth):
+    """A runtime enqueues call after call on one stream; the first kernels of a call start while the last ones of the
+    call before still run.  Every call's output has the bits of the same call run alone, with row counts, layers and
+    kernel forms (two-launch router, two-launch MLP, CUDA-core GEMM) changing from call to call."""
+    import torch
+    E, H, D = 16, 256, 320
+    blk = pkg.MoeBlock(H, D, E, n_layers=2, max_rows=2049)
+    try:
+        for i in range(2):
+            blk.load_layer(i, synth.make_layer(E, H, D, seed=71 + i))
+        calls = [(rows, flags, layer) for flags in (0, 4, 8, 1, 12) for rows in (2049, 1, 33, 513, 512) for layer in (0, 1)]
+        calls = [calls[i * 7 % len(calls)] for i in range(2 * len(calls))]
+        d_in = [torch.from_numpy(synth.make_tokens(2049, H, seed=80 + i).view(np.int16)).cuda() for i in range(3)]
+
+        def run(alone):
+            outs = [torch.zeros((rows, H), dtype=torch.int16, device="cuda") for rows, _, _ in calls]
+            s = torch.cuda.Stream()
+            torch.cuda.synchronize()
+            for i, ((rows, flags, layer), out) in enumerate(zip(calls, outs)):
+                blk.forward(layer, d_in[i % 3].data_ptr(), rows, out.data_ptr(), flags, s.cuda_stream)
+                if alone:
+                    s.synchronize()
+            blk.synchronize()
+            return outs
+
+        want, got = run(True), run(False)
+        for c, a, b in zip(calls, want, got):
+            assert torch.equal(a, b), c
+    finally:
+        blk.close()
+
+
+@pytest.mark.parametrize("rows", [1, 64, 700])
+def test_block_in_place_over_several_layers(rows, pkg, synth):
+    """The residual stream goes through the layers in place, with nothing between the calls: the bits of the same calls
+    run one at a time."""
+    import torch
+    E, H, D, L = 16, 256, 320, 3
+    blk = pkg.MoeBlock(H, D, E, n_layers=L, max_rows=rows)
+    try:
+        for i in range(L):
+            blk.load_layer(i, synth.make_layer(E, H, D, seed=90 + i))
+        x0 = torch.randn((rows, H), device="cuda").to(torch.bfloat16)
+        gains = [(1.0 + 0.25 * torch.randn(H, device="cuda")).to(torch.bfloat16) for _ in range(L)]
+
+        def run(alone):
+            x = x0.clone()
+            s = torch.cuda.Stream()
+            torch.cuda.synchronize()
+            for i in range(4 * L):
+                blk.block(i % L, x.data_ptr(), gains[i % L].data_ptr(), rows, stream=s.cuda_stream)
+                if alone:
+                    s.synchronize()
+            blk.synchronize()
+            return x.view(torch.int16)
+
+        assert torch.equal(run(True), run(False))
+    finally:
+        blk.close()
+
+
 def test_expert_output_beyond_fp16_is_reported(pkg, synth):
     """The per-(token, expert) MLP2 outputs wait for the combine in fp16; a magnitude above 65504 is an
     error code, not a silent infinity, and the handle keeps working."""
