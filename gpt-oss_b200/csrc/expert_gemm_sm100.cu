@@ -385,8 +385,10 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
       for (uint32_t spin = 0; published < mine; ++spin) {
         const uint32_t done = __reduce_min_sync(0xffffffffu, ld_acquire_cta(prog_base + 4u * (lane % kEpiWarps)));
         if (done > published) {
-          __threadfence();
+          // Each lane has acquired the progress of one epilogue warp; the warp barrier puts all sixteen before every
+          // lane's fence, and the fence before the counts that the lane adds: whoever acquires a count sees all rows.
           __syncwarp();
+          __threadfence();
           for (uint32_t i = published + lane; i < done; i += 32)
             atomicAdd(f.tile_done + pa.work[pair + static_cast<int>(i) * pairs].tile, 1u);
           if (lane == 0) atomicAdd(f.tile_done + f.total_slot, done - published);

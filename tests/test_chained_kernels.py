@@ -1,7 +1,12 @@
-"""Kernels that programmatic dependent launch may start early (they call grid_dep_wait or grid_dep_sync) read what
+"""Orderings that only a memory model shows: a compiler or a GPU that used the freedom would give rare wrong results and
+nothing a GPU test could be relied on to see, so the sources are checked.
+
+Kernels that programmatic dependent launch may start early (they call grid_dep_wait or grid_dep_sync) read what
 other kernels are still writing, so none of it may come through the read-only path: no __ldg, and no __restrict__ on
-anything but a layer's constants.  A compiler that moved such a load above the wait would show as rare wrong routing on
-a GPU and nowhere else, so the sources are checked."""
+anything but a layer's constants.
+
+The warp that counts finished MLP1 items publishes rows that sixteen other warps wrote: acquire in every lane, warp
+barrier, fence in every lane, then the counts."""
 import glob
 import os
 import re
@@ -27,3 +32,11 @@ def test_chained_kernels_read_with_ordinary_loads():
         restricted = set(re.findall(r"__restrict__ (\w+)", head + body))
         assert restricted <= CONSTANT, (name, restricted - CONSTANT)
         assert "__ldg(" not in body, name
+
+
+def test_counts_are_published_behind_all_epilogue_warps():
+    body = {n: b for n, _, b in kernels()}["expert_gemm_kernel"]
+    part = body[body.index("warp == kDoneWarp"):]
+    steps = ["ld_acquire_cta(", "__syncwarp();", "__threadfence();", "atomicAdd(f.tile_done + pa.work"]
+    at = [part.index(x) for x in steps]
+    assert at == sorted(at)
