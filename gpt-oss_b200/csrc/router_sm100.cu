@@ -135,7 +135,9 @@ router_kernel(const __grid_constant__ CUtensorMap tm_t, const __grid_constant__ 
       __syncwarp();
     }
   } else if (warp == 5) {
-    // ---- issue: 3 planes x 4 k steps of 16 per chunk, all into the same accumulator
+    // ---- issue: 3 planes x 4 k steps of 16 per chunk, all into the same accumulator.  No stage can be full before the
+    // producer has passed this wait; without it the bounded waits below would count the predecessor's time as theirs.
+    grid_dep_wait();
     const uint32_t idesc = idesc_bf16_m128(static_cast<uint32_t>(n_mma));
     for (int i = 0; i < n; ++i) {
       const int s = i % kRtStages;

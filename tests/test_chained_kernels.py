@@ -40,3 +40,17 @@ def test_counts_are_published_behind_all_epilogue_warps():
     steps = ["ld_acquire_cta(", "__syncwarp();", "__threadfence();", "atomicAdd(f.tile_done + pa.work"]
     at = [part.index(x) for x in steps]
     assert at == sorted(at)
+
+
+def test_no_bounded_wait_starts_before_the_predecessor_is_done():
+    """The ~1 s limit of a wait must not run while a kernel only waits for its turn: every role of the kernels with
+    bounded waits passes the grid wait first."""
+    body = {n: b for n, _, b in kernels()}
+    gemm = body["expert_gemm_kernel"]
+    assert gemm.index("grid_dep_sync();") < gemm.index("mbar_wait_warp(")
+    router = body["router_kernel"]
+    roles = re.split(r"(?:if|else if) \(warp (?:==|<) \d\) \{", router[router.index("grid_dep_release();"):])
+    roles = [r for r in roles[1:] if "mbar_wait_warp(" in r]
+    assert len(roles) == 3
+    for r in roles:
+        assert "grid_dep_wait();" in r and r.index("grid_dep_wait();") < r.index("mbar_wait_warp(")
