@@ -217,15 +217,18 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
       }
       const int half = (w.expert * n_ntiles + w.ntile) * 2 + rank;
       const uint8_t *tiles = w_tiles + static_cast<size_t>(half) * nkc * kWTileBytes;
-      // weights pass through once per step: they must not push the activations and the results out of L2
+      // weights pass through once per step: the loads leave them first in line to go, before activations and results
       for (int kc = 0; kc < nkc; kc += kSlices, tiles += 2 * kWTileBytes) {
         if (!mbar_wait_warp(empty_bar(s), e_par, abort_flag, status, ST_WAIT_EMPTY)) { ok = false; break; }
         const uint32_t stage = smem_base + s * kStageBytes;
         if (elect_one()) {
           // The ring alone holds less than HBM's latency takes at full rate (four stages turn round in ~2800 cycles):
-          // while one item streams, the next one's weights come into L2.  The whole launch, 128 experts: 32 rows
-          // 174 -> 162 us (HBM at its peak), 256 rows 299 -> 279, 1856 rows 396 -> 375.  Only the first of the items
-          // that share a weight block does it: done by all of them it cost 4-8 % at 4 tiles per expert.
+          // while one item streams, the next one's weights come into L2.  It pays where HBM is the bound, that is for
+          // experts with a single token tile (WorkItem::lead).  Whole calls, us, without it / for experts of one tile /
+          // for the first tile of every expert: 1 row 41.6 / 39.2 / 39.3, 32 rows 195.5 / 185.1 / 184.9, 256 rows (block)
+          // 338 / 328 / 327, 1856 rows 528 / 520 / 523; two tiles (32 experts, 1536 rows, block) 344 / 344 / 361; three
+          // (8192 rows) 1824 / 1816 / 1895.  Experts of up to two tiles: 354 at two.  The evict-first policy of the
+          // loads changes nothing here, neither the times nor the ~5 MB more that DRAM is written (464 rows, 32 experts).
           if (ahead != nullptr && kc < ahead_nkc)
             bulk_prefetch_l2(ahead + static_cast<size_t>(kc) * kWTileBytes, min(2, ahead_nkc - kc) * kWTileBytes);
           if (kc + 1 < nkc) {

@@ -116,7 +116,7 @@ struct __align__(16) WorkItem {
   int tile;    // global token-tile index
   int row0;    // first permuted row of the token tile
   int ntok;    // token rows in the tile (1..kMaxTileTok)
-  int lead;    // 1 for the first of the items that share a weight block: it brings the block into L2
+  int lead;    // 1 for the one item of its weight block (the expert has one token tile): the block is brought into L2 ahead
   int pad[2];
 };
 

@@ -211,7 +211,7 @@ build_index_kernel(const int *topk_idx, const int *hist, int *counts, int T, int
       it.tile = tiles_before + tt;
       it.row0 = off + tt * per_tile;
       it.ntok = min(per_tile, cnt - tt * per_tile);
-      it.lead = tt == 0;
+      it.lead = ntt == 1;
       it.pad[0] = it.pad[1] = 0;
       if (start + i < cap) work[start + i] = it;
       else atomicOr(status, ST_BAD_INDEX);
