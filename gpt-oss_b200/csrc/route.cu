@@ -100,9 +100,14 @@ void launch_topk_softmax(float *logits, const float *partial, int splits, const 
 // route_build_index_kernel_bf16wts (kernels/moe.hpp:1173-1270): rows of one
 // expert are in ascending token order.
 // ---------------------------------------------------------------------------
-// kK: experts per token known at compile time, 0: any.  The loops are kept rolled: at small batches this kernel, like the
-// quantiser below, takes as long as its instructions take to arrive (each layer's weights push the code out of the caches).
-template <int kK>
+// kK: experts per token known at compile time, 0: any.  Two forms, by the rows of the batch as in the quantiser below:
+//  * up to kFewRows rows (kHeld = 0): rolled loops, every selection read twice.  This kernel then takes as long as its
+//    instructions take to arrive (each layer's weights push the code out of the caches).
+//  * above (kHeld = 8): a warp's first eight ballot steps are loaded together and stay in registers for the second walk.
+//    Kernel alone, us, rolled / held: 600 rows 6.5 / 6.4, 1536 rows of 32 experts 8.4 / 7.8, 1856 rows 9.8 / 9.0, 3000 rows
+//    9.0 / 8.7, 7424 rows 13.0 / 11.9, 8192 rows 13.1 / 11.9.
+constexpr int kFewRows = 512;
+template <int kK, int kHeld>
 __global__ void __launch_bounds__(1024)
 build_index_kernel(const int *topk_idx, const int *hist, int *counts, int T, int E, int K, int n_ntiles1, int n_ntiles2,
                    int *offsets, int *tile_base, int *pair_row, int *row_token, int2 *pair_slot, unsigned int *tile_done,
@@ -112,11 +117,11 @@ build_index_kernel(const int *topk_idx, const int *hist, int *counts, int T, int
   __shared__ int s_warp[32];
   grid_dep_sync();
   const int e = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_warps = blockDim.x >> 5;   // 8, or 32 for batches whose selections 8 warps cannot hold in registers
+  const int n_warps = blockDim.x >> 5;   // 8, or 32 above the 2048 rows whose selections 8 warps hold in registers
 
   // Stable compaction in ascending token order.  Warp w owns the contiguous token range [w*per, (w+1)*per):
   // a first walk counts the range's hits with ballots, the block's one barrier turns the warps' counts into
-  // starting positions, a second walk (its loads hit L1) writes the rows.
+  // starting positions, a second walk writes the rows.
   const int per = ((T + n_warps - 1) / n_warps + 31) / 32 * 32;       // tokens per warp, whole ballot steps
   const int t_begin = warp * per, t_end = min(T, t_begin + per);
   auto hit_of = [&](int t) -> int {
@@ -131,9 +136,15 @@ build_index_kernel(const int *topk_idx, const int *hist, int *counts, int T, int
       return -1;
     }
   };
+  int held[kHeld > 0 ? kHeld : 1];
+#pragma unroll
+  for (int j = 0; j < kHeld; ++j) held[j] = hit_of(t_begin + 32 * j + lane);
+  const int t_rest = t_begin + 32 * kHeld;   // what is not held
   int mine = 0;
+  if constexpr (kHeld == 0) {
 #pragma unroll 4
-  for (int t0 = t_begin; t0 < t_end; t0 += 32) mine += __popc(__ballot_sync(0xffffffffu, hit_of(t0 + lane) >= 0));
+    for (int t0 = t_rest; t0 < t_end; t0 += 32) mine += __popc(__ballot_sync(0xffffffffu, hit_of(t0 + lane) >= 0));
+  }
 
   // exclusive prefix over experts below e: rows and token tiles (its loads travel with the ones above)
   int my_rows = 0, my_tiles = 0;
@@ -147,6 +158,12 @@ build_index_kernel(const int *topk_idx, const int *hist, int *counts, int T, int
   for (int off = 16; off; off >>= 1) {
     my_rows += __shfl_xor_sync(0xffffffffu, my_rows, off);
     my_tiles += __shfl_xor_sync(0xffffffffu, my_tiles, off);
+  }
+  if constexpr (kHeld > 0) {   // behind the loads of the prefix, so that both are in flight together
+#pragma unroll
+    for (int j = 0; j < kHeld; ++j) mine += __popc(__ballot_sync(0xffffffffu, held[j] >= 0));
+#pragma unroll 4
+    for (int t0 = t_rest; t0 < t_end; t0 += 32) mine += __popc(__ballot_sync(0xffffffffu, hit_of(t0 + lane) >= 0));
   }
   if (lane == 0) { s_red[0][warp] = my_rows; s_red[1][warp] = my_tiles; s_warp[warp] = mine; }
   __syncthreads();   // the only block-wide barrier: prefix partials and hit counts of all warps
@@ -190,8 +207,10 @@ build_index_kernel(const int *topk_idx, const int *hist, int *counts, int T, int
     }
     before += __popc(m);
   };
+#pragma unroll
+  for (int j = 0; j < kHeld; ++j) place(t_begin + 32 * j + lane, held[j]);
 #pragma unroll 1
-  for (int t0 = t_begin; t0 < t_end; t0 += 32) place(t0 + lane, hit_of(t0 + lane));
+  for (int t0 = t_rest; t0 < t_end; t0 += 32) place(t0 + lane, hit_of(t0 + lane));
   if (tid == 0 && total_hits != cnt) atomicOr(status, ST_BAD_INDEX);
 
   // work items: one per (token tile, block of kBlockRows weight rows); items that share a
@@ -224,9 +243,11 @@ void launch_build_index(const int *topk_idx, const int *hist, int *counts, int T
                         int *offsets, int *tile_base, int *pair_row, int *row_token, int2 *pair_slot,
                         unsigned int *tile_done, int tile_done_total_slot, WorkItem *work1, WorkItem *work2, int *n_work, int max_work1, int max_work2,
                         unsigned int *status, cudaStream_t s, bool chained) {
-  launch_kernel(K == 4 ? build_index_kernel<4> : build_index_kernel<0>, dim3(E), T > 2048 ? 1024 : 256, 0, s, chained, 0, topk_idx, hist, counts, T, E, K, n_ntiles1,
-                n_ntiles2, offsets, tile_base, pair_row, row_token, pair_slot, tile_done, tile_done_total_slot, work1, work2,
-                n_work, max_work1, max_work2, status);
+  auto kernel = T <= kFewRows ? (K == 4 ? build_index_kernel<4, 0> : build_index_kernel<0, 0>)
+                                : (K == 4 ? build_index_kernel<4, 8> : build_index_kernel<0, 8>);
+  launch_kernel(kernel, dim3(E), T > 2048 ? 1024 : 256, 0, s, chained, 0, topk_idx, hist, counts, T, E, K,
+                n_ntiles1, n_ntiles2, offsets, tile_base, pair_row, row_token, pair_slot, tile_done, tile_done_total_slot,
+                work1, work2, n_work, max_work1, max_work2, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -243,14 +264,13 @@ void launch_build_index(const int *topk_idx, const int *hist, int *counts, int T
 // ---------------------------------------------------------------------------
 // The two rows depend on the token only, not on the expert, so a warp quantises one TOKEN and stores the result once per
 // selected expert, at the tile rows build_index_kernel assigned to the (token, expert) pairs.  Two forms:
-//  * up to kQrFewRows rows: rolled loops, two passes over the row (the second out of L1), 9 KB of code.  A small batch
+//  * up to kFewRows rows: rolled loops, two passes over the row (the second out of L1), 9 KB of code.  A small batch
 //    waits for the code to be fetched (each layer's weights push it out of the caches), and that is most of the kernel's
 //    time: with the 52 KB of the other form, and an index kernel twice the size, a call with 1 row took 45.2 us instead of
 //    39.3, 32 rows 186.7 / 184.5, 256 rows (block) 331 / 327.
 //  * larger batches: the row stays in registers (kQrVec x 32 bytes per lane), bound by the writes; the rolled form takes
 //    46 us instead of 41 at 7424 rows, and the same at 1536.
 constexpr int kQrWarps = 4;
-constexpr int kQrFewRows = 512;
 
 template <int kQrVec>         // 6: rows of up to 3072 elements, 8: up to 4096
 __global__ void __launch_bounds__(kQrWarps * 32)
@@ -420,7 +440,7 @@ int quantize_rows_max_hidden() { return 32 * 8 * 16; }
 void launch_quantize_rows(const __nv_bfloat16 *t, const int2 *pair_slot, int T, int K, uint8_t *xq, uint8_t *sfb, int H,
                           cudaStream_t s, bool chained) {
   const int blocks = (T + kQrWarps - 1) / kQrWarps;
-  auto kernel = T <= kQrFewRows ? (K == 4 ? quantize_few_rows_kernel<4> : quantize_few_rows_kernel<0>)
+  auto kernel = T <= kFewRows ? (K == 4 ? quantize_few_rows_kernel<4> : quantize_few_rows_kernel<0>)
                                 : (H <= 32 * 6 * 16 ? quantize_rows_kernel<6> : quantize_rows_kernel<8>);
   launch_kernel(kernel, dim3(blocks), kQrWarps * 32, 0, s, chained,
                 0, t, pair_slot, T, K, xq, sfb, H);

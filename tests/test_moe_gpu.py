@@ -170,6 +170,27 @@ def test_routing_invariants(pkg, synth):
         blk.close()
 
 
+@pytest.mark.parametrize("top_k", [3, 4])
+@pytest.mark.parametrize("T", [511, 512, 513, 2047, 2048, 2049, 8192, 8225])
+def test_index_at_the_edges_of_its_forms(T, top_k, pkg, synth):
+    """Rolled up to 512 rows, selections in registers above; 8 warps up to 2048 rows, 32 above; past 8192 rows a warp's
+    range is longer than what it holds.  The permutation is a stable sort of the selections, exactly."""
+    E, H, D = 16, 64, 32
+    blk = pkg.MoeBlock(H, D, E, top_k=top_k, max_rows=T)
+    try:
+        blk.load_layer(0, synth.make_layer(E, H, D, seed=13, zipf_s=1.2))
+        blk.forward_host(0, synth.make_tokens(T, H, seed=T))
+        idx = blk.debug(pkg.DBG_TOPK_IDX)
+        order = np.argsort(idx.ravel(), kind="stable")    # by expert, then token (an expert has a token once)
+        want = np.empty(T * top_k, dtype=np.int32)
+        want[order] = np.arange(T * top_k)
+        assert np.array_equal(blk.debug(pkg.DBG_PAIR_ROW).ravel(), want)
+        assert np.array_equal(blk.debug(pkg.DBG_ROW_TOKEN), order // top_k)
+        assert np.array_equal(blk.debug(pkg.DBG_COUNTS), np.bincount(idx.ravel(), minlength=E))
+    finally:
+        blk.close()
+
+
 @pytest.mark.parametrize("E,H,D,T,zipf", [
     (8, 128, 128, 5, None),      # fewer rows than one MMA column group
     (8, 256, 192, 100, None),    # K tail (192 = 128 + 64), ragged counts
