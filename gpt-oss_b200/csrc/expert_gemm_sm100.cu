@@ -26,15 +26,19 @@
 // Per 128-element slice of k (two to a shared-memory stage) each CTA loads: weight codes
 // [120 rows x 128] (TMA, 16U4_ALIGN16B: 4-bit codes are expanded to the 8-bit containers the
 // MMA reads, 128-byte swizzle), their 512-byte scale atom (pre-tiled at load time), and its
-// half of the token rows.  The weights of both slices are one TMA box, the token rows one plain bulk
-// copy (the quantiser and the SwiGLU epilogue write them interleaved by slice and with the 128-byte
+// half of the token rows.  The weights of both slices are one TMA box, and so are the token rows (the
+// quantiser and the SwiGLU epilogue write them interleaved by slice and with the 128-byte
 // swizzle already applied): what a role spends per stage is issue time, ~150 cycles per copy, ~110
 // per wait, ~35 per commit, and it was that time that bounded earlier forms with one slice per stage.
 // Two producer warps (weights and their scales; tokens) keep kStages stages in flight.  The MMA warp
 // of the even CTA copies the scales of both CTAs to tensor memory (tcgen05.cp) and issues four
-// instructions per slice for the pair; the
-// same warp of the odd CTA reports each stage that has landed in its shared memory to the even
-// one.  Issuing warps stay converged and elect one lane, so that descriptors and
+// instructions per slice for the pair.  The copies of both CTAs complete on the even CTA's barrier (loads of
+// cta_group::2, whose completion is a release at cluster scope), where its MMA warp acquires them at cluster scope.
+// (The odd CTA used to report what had landed with an arrival of CTA scope, which promises nothing across CTAs; with
+// release at cluster scope such a report costs 0.9 us a stage.  Whole calls, us, report of CTA scope / now / now but with
+// the acquire left out: 1 row 39.4 / 39.2 / 39.0, 32 rows 185.2 / 186.2 / 184.5, 64 rows of 32 experts 102.9 / 103.9 /
+// 103.1, 256 rows (block) 330 / 332 / 330, larger ones within the spread of the runs.)
+// Issuing warps stay converged and elect one lane, so that descriptors and
 // tensor-memory addresses live in uniform registers.  Sixteen epilogue warps per CTA drain the
 // fp32 accumulator (double buffered: 2 x 192 columns).
 // One more warp counts finished MLP1 items for the MLP2 items that wait for them.
@@ -128,9 +132,8 @@ __device__ __forceinline__ void transpose_pair(uint32_t &w0, uint32_t &w1, int q
 // producers run ahead of that wait.  MLP1 items wait for nothing and every pair is resident (the grid is
 // what the device places at once), so the MLP2 waits always end.
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__ CUtensorMap tm_w1_last,
-                   const __grid_constant__ CUtensorMap tm_w2, const __grid_constant__ CUtensorMap tm_w2_last, const GemmArgs pa,
-                   const GemmArgs pb, const MlpFuse f) {
+expert_gemm_kernel(const __grid_constant__ WeightMaps tm_w1, const __grid_constant__ WeightMaps tm_w2,
+                   const __grid_constant__ TokenMaps tm_x, const GemmArgs pa, const GemmArgs pb, const MlpFuse f) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -148,8 +151,8 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
   const int rank = static_cast<int>(cluster_ctarank());   // 0 issues the MMAs of the pair
 
   if (threadIdx.x == 0) {
-    // full: both producers; in the even CTA also the report that the odd CTA's half has landed
-    for (int s = 0; s < kStages; ++s) { mbar_init(full_bar(s), rank == 0 ? 3 : 2); mbar_init(empty_bar(s), 1); }
+    // full (used in the even CTA only): its producers, which announce the bytes of both CTAs
+    for (int s = 0; s < kStages; ++s) { mbar_init(full_bar(s), 2); mbar_init(empty_bar(s), 1); }
     for (int d = 0; d < 2; ++d) {
       mbar_init(dfull_bar(d), 1);
       mbar_init(dempty_bar(d), 2 * kEpiWarps);   // the epilogue warps of both CTAs (even CTA's copy only)
@@ -164,8 +167,9 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
     tmem_relinquish_pair();
   }
   if (warp == kWProducerWarp && lane == 0) {
-    if (f.phase_begin == 0) { prefetch_tensormap(&tm_w1); prefetch_tensormap(&tm_w1_last); }
-    if (f.phase_end == 2) { prefetch_tensormap(&tm_w2); prefetch_tensormap(&tm_w2_last); }
+    const WeightMaps *m = f.phase_begin == 0 ? &tm_w1 : &tm_w2;
+    prefetch_tensormap(&m->codes);
+    prefetch_tensormap(&m->scales);
   }
   tc_fence_before();
   __syncthreads();
@@ -184,6 +188,9 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
   };
   unsigned int *status = pa.status;
   bool ok = true;
+  // The even CTA's full barriers.  A copy of the odd CTA for the next round of a stage cannot come early: it waits for the
+  // MMAs of this round, which wait for the barrier's phase.
+  const uint32_t full0 = map_to_cta(full_bar(0), 0);
 
   if (warp == kWProducerWarp) {
     // ------------------------------------------------------------- weight producer
@@ -191,7 +198,7 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
     const uint64_t w_policy = l2_policy_evict_first();
    for (int phase = f.phase_begin; ok && phase < f.phase_end; ++phase) {
     const bool second = phase != 0;
-    const CUtensorMap *tm_w = second ? &tm_w2 : &tm_w1, *tm_last = second ? &tm_w2_last : &tm_w1_last;
+    const WeightMaps *tm_w = second ? &tm_w2 : &tm_w1;
     const WorkItem *work = second ? pb.work : pa.work;
     const int n_work = second ? *pb.n_work : n_work1;
     const int nkc = second ? pb.n_kchunks : pa.n_kchunks, n_ntiles = second ? pb.n_ntiles : pa.n_ntiles;
@@ -216,10 +223,9 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
         }
       }
       const int half = (w.expert * n_ntiles + w.ntile) * 2 + rank;
-      const uint8_t *tiles = w_tiles + static_cast<size_t>(half) * nkc * kWTileBytes;
       // weights pass through once per step: the loads leave them first in line to go, before activations and results
-      for (int kc = 0; kc < nkc; kc += kSlices, tiles += 2 * kWTileBytes) {
-        if (!mbar_wait_warp(empty_bar(s), e_par, abort_flag, status, ST_WAIT_EMPTY)) { ok = false; break; }
+      for (int kc = 0; kc < nkc; kc += kSlices) {
+        if (!mbar_wait_warp<Wait::kClusterRelaxed>(empty_bar(s), e_par, abort_flag, status, ST_WAIT_EMPTY)) { ok = false; break; }
         const uint32_t stage = smem_base + s * kStageBytes;
         if (elect_one()) {
           // The ring alone holds less than HBM's latency takes at full rate (four stages turn round in ~2800 cycles):
@@ -231,14 +237,14 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
           // loads changes nothing here, neither the times nor the ~5 MB more that DRAM is written (464 rows, 32 experts).
           if (ahead != nullptr && kc < ahead_nkc)
             bulk_prefetch_l2(ahead + static_cast<size_t>(kc) * kWTileBytes, min(2, ahead_nkc - kc) * kWTileBytes);
+          if (rank == 0) mbar_arrive_expect_tx(full_bar(s), 2 * min(2, nkc - kc) * (kWLoadBytes + kSfAtomBytes));
+          const uint32_t bar = full0 + 8u * s;
           if (kc + 1 < nkc) {
-            mbar_arrive_expect_tx(full_bar(s), 2 * (kWLoadBytes + kSfAtomBytes));
-            tma_load_5d_hint(stage, tm_w, 0, 0, 0, kc >> 1, half, full_bar(s), w_policy);
-            bulk_load_hint(stage + kSfaOff, tiles + 2 * kWTileCodes, 2 * kSfAtomBytes, full_bar(s), w_policy);
+            tma_load_5d_pair_hint(stage, &tm_w->codes, 0, 0, 0, kc >> 1, half, bar, w_policy);
+            tma_load_3d_pair_hint(stage + kSfaOff, &tm_w->scales, 0, kc >> 1, half, bar, w_policy);
           } else {
-            mbar_arrive_expect_tx(full_bar(s), kWLoadBytes + kSfAtomBytes);
-            tma_load_3d_hint(stage, tm_last, 0, 0, half, full_bar(s), w_policy);
-            bulk_load_hint(stage + kSfaOff, tiles + kWTileCodes, kSfAtomBytes, full_bar(s), w_policy);
+            tma_load_3d_pair_hint(stage, &tm_w->codes_last, 0, 0, half, bar, w_policy);
+            tma_load_2d_pair_hint(stage + kSfaOff, &tm_w->scales_last, 0, half, bar, w_policy);
           }
         }
         if (++s == kStages) { s = 0; e_par ^= 1u; }
@@ -254,8 +260,8 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
     const WorkItem *work = second ? pb.work : pa.work;
     const int n_work = second ? *pb.n_work : n_work1;
     const int nkc = second ? pb.n_kchunks : pa.n_kchunks;
-    const uint8_t *xq = second ? pb.xq : pa.xq, *sfb = second ? pb.sfb : pa.sfb;
-    const int sfb_tile_stride = second ? pb.sfb_tile_stride : pa.sfb_tile_stride;
+    const int x_half0 = second ? pb.x_half0 : pa.x_half0;
+    const int sfb_tile0 = second ? pb.sfb_tile0 : pa.sfb_tile0, sfb_step = second ? pb.sfb_step : pa.sfb_step;
     const int first = first_item(phase);
     WorkItem w_next = {};
     if (first < n_work) w_next = work[first];
@@ -285,35 +291,25 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
         asm volatile("fence.proxy.async;" ::: "memory");
       }
       // this CTA's half of the tile's rows (both slices of a pair; of a single last slice the unused other half too)
-      const uint32_t bytes = static_cast<uint32_t>(tile_n(w.ntok)) * kChunkK;
-      const uint8_t *src = xq + static_cast<size_t>(w.tile) * slice_pairs(nkc) * kPairBytes + rank * (kPairBytes / 2);
-      for (int kc = 0; kc < nkc; kc += kSlices, src += kPairBytes) {
-        if (!mbar_wait_warp(empty_bar(s), e_par, abort_flag, status, ST_WAIT_EMPTY)) { ok = false; break; }
+      const int n_rows = tile_n(w.ntok);
+      const uint32_t bytes = static_cast<uint32_t>(n_rows) * kChunkK;
+      const CUtensorMap *tm_rows = &tm_x.rows[n_rows / 16 - 1];
+      const int half = x_half0 + w.tile * slice_pairs(nkc) * 2 + rank;
+      for (int kc = 0; kc < nkc; kc += kSlices) {
+        if (!mbar_wait_warp<Wait::kClusterRelaxed>(empty_bar(s), e_par, abort_flag, status, ST_WAIT_EMPTY)) { ok = false; break; }
         const uint32_t stage = smem_base + s * kStageBytes;
         if (elect_one()) {
-          mbar_arrive_expect_tx(full_bar(s), bytes + (kc == 0 ? kSfbTileBytes : 0));
-          if (kc == 0)
-            bulk_load(stage + kSfbOff, sfb + static_cast<size_t>(w.tile) * sfb_tile_stride, kSfbTileBytes, full_bar(s));
-          bulk_load(stage + kXOff, src, bytes, full_bar(s));
+          if (rank == 0) mbar_arrive_expect_tx(full_bar(s), 2 * (bytes + (kc == 0 ? kSfbTileBytes : 0)));
+          const uint32_t bar = full0 + 8u * s;
+          if (kc == 0) tma_load_2d_pair(stage + kSfbOff, &tm_x.scales, 0, sfb_tile0 + w.tile * sfb_step, bar);
+          tma_load_3d_pair(stage + kXOff, tm_rows, 0, 0, half + kc, bar);   // a pair of slices has two halves
         }
         if (++s == kStages) { s = 0; e_par ^= 1u; }
       }
     }
    }
   } else if (warp == kMmaWarp && rank != 0) {
-    // ------------------------------------------------------------- odd CTA: report landed slices to the even one
-    uint32_t s = 0, f_par = 0;
-   for (int phase = f.phase_begin; ok && phase < f.phase_end; ++phase) {
-    const bool second = phase != 0;
-    const int n_work = second ? *pb.n_work : n_work1;
-    const int nkc = second ? pb.n_kchunks : pa.n_kchunks;
-    for (int wi = first_item(phase); ok && wi < n_work; wi += pairs)
-      for (int kc = 0; kc < nkc; kc += kSlices) {
-        if (!mbar_wait_warp(full_bar(s), f_par, abort_flag, status, ST_WAIT_FULL)) { ok = false; break; }
-        if (elect_one()) mbar_arrive_cluster(full_bar(s), 0);
-        if (++s == kStages) { s = 0; f_par ^= 1u; }
-      }
-   }
+    // the even CTA's warp issues for both
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------- even CTA: MMA issuer of the pair
     // The warp stays converged and one elected lane issues the tcgen05 instructions, so that their operands
@@ -335,7 +331,7 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
       const uint32_t n = __shfl_sync(0xffffffffu, static_cast<uint32_t>(tile_n(ntok_next)), 0);
       if (wi + pairs < n_work) ntok_next = work[wi + pairs].ntok;
       const uint32_t d = item & 1u;
-      if (!mbar_wait_warp(dempty_bar(d), ((item >> 1) & 1u) ^ 1u, abort_flag, status, ST_WAIT_DEMPTY)) { ok = false; break; }
+      if (!mbar_wait_warp<Wait::kClusterRelaxed>(dempty_bar(d), ((item >> 1) & 1u) ^ 1u, abort_flag, status, ST_WAIT_DEMPTY)) { ok = false; break; }
       tc_fence_after();
       const uint32_t sfb_t = tm + kSfbCol0 + 8 * d;
       const uint32_t d_addr = tm + d * kAccBufCols;
@@ -356,7 +352,7 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
         }
       };
       for (int kc = 0; kc < nkc; kc += kSlices) {
-        if (!mbar_wait_warp(full_bar(s), f_par, abort_flag, status, ST_WAIT_FULL)) { ok = false; break; }
+        if (!mbar_wait_warp<Wait::kCluster>(full_bar(s), f_par, abort_flag, status, ST_WAIT_FULL)) { ok = false; break; }
         const uint32_t stage = smem_base + s * kStageBytes;
         if (elect_one()) {
           if (kc == 0) {
@@ -416,6 +412,7 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
     const int odd = lane & 1;
     const int lrow = quad * 32 + lane, q4 = (lane >> 1) & 3;
     const float h_scale = exp2f(static_cast<float>(-pa.h_exp));
+    const uint32_t dempty0 = map_to_cta(dempty_bar(0), 0);
     uint32_t item = 0;
    for (int phase = f.phase_begin; ok && phase < f.phase_end; ++phase) {
     const bool second = phase != 0;
@@ -435,13 +432,13 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
       const bool row_ok = lrow < kHalfRows && n0 + lrow < R;
       const float b = row_ok && add_bias ? __bfloat162float(bias[static_cast<size_t>(w.expert) * R + n0 + lrow]) : 0.f;
       const int n_chunks = tile_n(w.ntok) / 16;   // 8 tokens each, and as many 4-token groups per CTA
-      if (!mbar_wait_warp(dfull_bar(d), (item >> 1) & 1u, abort_flag, status, ST_WAIT_DFULL)) { ok = false; break; }
+      if (!mbar_wait_warp<Wait::kClusterRelaxed>(dfull_bar(d), (item >> 1) & 1u, abort_flag, status, ST_WAIT_DFULL)) { ok = false; break; }
       tc_fence_after();
       const uint32_t acc = tmem_base + lane_field + d * kAccBufCols;
       auto release = [&]() {   // the accumulator is in registers (or not this warp's business): the MMAs may go on
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(dempty_bar(d), 0);
+        if (lane == 0) mbar_arrive_relaxed_cluster(dempty0 + 8u * d);
       };
       auto process = [&](const uint32_t (&v)[16], int c) {
         // Sum of the high and low partial products, plus the bias of this lane's row.  Of a pair of lanes (rows
@@ -518,7 +515,7 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_const
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();   // neither CTA leaves while the pair's MMAs or reports may still touch its memory
+  cluster_sync_all();   // neither CTA leaves while the pair's MMAs, copies or reports may still touch its memory
   if (warp == kMmaWarp) {
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, kTmemCols);
@@ -551,9 +548,9 @@ cudaError_t expert_gemm_init(int *grid) {
 
 // Phases [f.phase_begin, f.phase_end) of the expert MLP in one launch: both in the usual call, one at a
 // time (two launches, f.tile_done = nullptr) on request.
-void launch_expert_mlp(const CUtensorMap (&tm_w1)[2], const GemmArgs &a, const CUtensorMap (&tm_w2)[2], const GemmArgs &b,
-                       const MlpFuse &f, int grid, cudaStream_t s, bool chained) {
-  launch_kernel(expert_gemm_kernel, dim3(grid), kThreads, kSmemBytes, s, chained, 0, tm_w1[0], tm_w1[1], tm_w2[0], tm_w2[1], a, b, f);
+void launch_expert_mlp(const WeightMaps &tm_w1, const GemmArgs &a, const WeightMaps &tm_w2, const GemmArgs &b,
+                       const TokenMaps &tm_x, const MlpFuse &f, int grid, cudaStream_t s, bool chained) {
+  launch_kernel(expert_gemm_kernel, dim3(grid), kThreads, kSmemBytes, s, chained, 0, tm_w1, tm_w2, tm_x, a, b, f);
 }
 
 int expert_mlp_done_per_tile(int n_ntiles1) { return 2 * n_ntiles1; }

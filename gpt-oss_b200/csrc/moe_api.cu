@@ -37,30 +37,56 @@ int fail(moe_ctx *c, int code, const char *fmt, ...) {
                   "%s failed: %s (%s:%d)", #expr, cudaGetErrorString(e__), __FILE__, __LINE__); \
   } while (0)
 
-// Tensor maps of the weight codes (LayerWeights::w1_tiles), declared to TMA as 4-bit elements that it expands to the
-// 8-bit containers of the block-scaled MMA (16U4_ALIGN16B).  m[0]: one box = the codes of a pair of k slices, a
-// contiguous 15 KB read; m[1]: the codes of the single last slice of an odd number.  A map of slices that do not
-// exist is made with one of them and never used.
-int make_weight_maps(moe_ctx *c, CUtensorMap (&m)[2], const uint8_t *base, size_t n_halves, int n_kc) {
+// A tensor map of contiguous rows of `inner` elements: dims and box without the innermost dimension, strides in bytes.
+CUresult encode_map(CUtensorMap *m, CUtensorMapDataType type, const uint8_t *base, int rank, cuuint64_t inner,
+                    const cuuint64_t (&dims)[4], const cuuint64_t (&strides)[4], const cuuint32_t (&box)[4],
+                    CUtensorMapSwizzle swizzle) {
   TensorMapEncodeFn fn = tensor_map_encoder();
-  if (!fn) return fail(c, MOE_ERR_CUDA, "cuTensorMapEncodeTiled not available");
-  const cuuint64_t half = static_cast<cuuint64_t>(n_kc) * kWTileBytes;
+  if (!fn) return CUDA_ERROR_NOT_FOUND;
+  const cuuint64_t d[5] = {inner, dims[0], dims[1], dims[2], dims[3]};
+  const cuuint32_t b[5] = {static_cast<cuuint32_t>(inner), box[0], box[1], box[2], box[3]};
   const cuuint32_t es[5] = {1, 1, 1, 1, 1};
-  const cuuint64_t dims0[5] = {kChunkK, kHalfRows, 2, static_cast<cuuint64_t>(std::max(1, n_kc / 2)), n_halves};
-  const cuuint64_t strides0[4] = {kChunkK / 2, kWTileCodes, 2 * kWTileBytes, half};
-  const cuuint32_t box0[5] = {kChunkK, kHalfRows, 2, 1, 1};
-  CUresult r = fn(&m[0], CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 5, const_cast<uint8_t *>(base), dims0, strides0, box0, es,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r == CUDA_SUCCESS) {
-    const cuuint64_t dims1[3] = {kChunkK, kHalfRows, n_halves};
-    const cuuint64_t strides1[2] = {kChunkK / 2, half};
-    const cuuint32_t box1[3] = {kChunkK, kHalfRows, 1};
-    r = fn(&m[1], CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3, const_cast<uint8_t *>(base) + w_codes_offset((n_kc - 1) & ~1),
-           dims1, strides1, box1, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  }
+  return fn(m, type, rank, const_cast<uint8_t *>(base), d, strides, b, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+}
+
+// Tensor maps of a weight matrix (LayerWeights::w1_tiles).  The codes are declared to TMA as 4-bit elements that it
+// expands to the 8-bit containers of the block-scaled MMA (16U4_ALIGN16B), the scale atoms as plain words.  A box is a
+// contiguous read: the codes (15 KB) or scales (1 KB) of a pair of k slices, or of the single last slice of an odd number.
+// A map of slices that do not exist is made with one of them and never used.
+int make_weight_maps(moe_ctx *c, WeightMaps &m, const uint8_t *base, size_t n_halves, int n_kc) {
+  const CUtensorMapDataType u4 = CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, u32 = CU_TENSOR_MAP_DATA_TYPE_UINT32;
+  const cuuint64_t half = static_cast<cuuint64_t>(n_kc) * kWTileBytes, pairs = std::max(1, n_kc / 2), nh = n_halves;
+  const int last = (n_kc - 1) & ~1;
+  CUresult r = encode_map(&m.codes, u4, base, 5, kChunkK, {kHalfRows, 2, pairs, nh},
+                          {kChunkK / 2, kWTileCodes, 2 * kWTileBytes, half}, {kHalfRows, 2, 1, 1}, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r == CUDA_SUCCESS)
+    r = encode_map(&m.scales, u32, base + 2 * kWTileCodes, 3, 2 * kSfAtomBytes / 4, {pairs, nh}, {2 * kWTileBytes, half}, {1, 1},
+                   CU_TENSOR_MAP_SWIZZLE_NONE);
+  if (r == CUDA_SUCCESS)
+    r = encode_map(&m.codes_last, u4, base + w_codes_offset(last), 3, kChunkK, {kHalfRows, nh}, {kChunkK / 2, half}, {kHalfRows, 1},
+                   CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r == CUDA_SUCCESS)
+    r = encode_map(&m.scales_last, u32, base + w_scales_offset(last, n_kc), 2, kSfAtomBytes / 4, {nh}, {half}, {1},
+                   CU_TENSOR_MAP_SWIZZLE_NONE);
   if (r != CUDA_SUCCESS) return fail(c, MOE_ERR_CUDA, "cuTensorMapEncodeTiled(weights, %zu x %d slices) -> %d", n_halves, n_kc, (int)r);
+  return MOE_OK;
+}
+
+// Tensor maps of the token rows (TokenMaps): n_halves halves at rows, n_tiles pairs of scale atoms at scales.
+int make_token_maps(moe_ctx *c, TokenMaps &m, const uint8_t *rows, size_t n_halves, const uint8_t *scales, size_t n_tiles) {
+  constexpr int kGroup = 2 * 8 * kChunkK;   // bytes of a group of 8 rows of both slices
+  static_assert(kGroup / 8 <= 256, "innermost extent of a box");
+  constexpr int kGroups = kPairBytes / 2 / kGroup;
+  static_assert(kGroups == sizeof(m.rows) / sizeof(m.rows[0]), "a map for every number of groups");
+  CUresult r = CUDA_SUCCESS;
+  for (int g = 1; g <= kGroups && r == CUDA_SUCCESS; ++g)
+    r = encode_map(&m.rows[g - 1], CU_TENSOR_MAP_DATA_TYPE_UINT64, rows, 3, kGroup / 8, {kGroups, n_halves}, {kGroup, kPairBytes / 2},
+                   {static_cast<cuuint32_t>(g), 1}, CU_TENSOR_MAP_SWIZZLE_NONE);
+  if (r == CUDA_SUCCESS)
+    r = encode_map(&m.scales, CU_TENSOR_MAP_DATA_TYPE_UINT32, scales, 2, kSfbTileBytes / 4, {n_tiles}, {kSfbTileBytes}, {1},
+                   CU_TENSOR_MAP_SWIZZLE_NONE);
+  if (r != CUDA_SUCCESS) return fail(c, MOE_ERR_CUDA, "cuTensorMapEncodeTiled(token rows, %zu halves) -> %d", n_halves, (int)r);
   return MOE_OK;
 }
 
@@ -259,27 +285,27 @@ int forward_impl(moe_ctx *c, int layer, const __nv_bfloat16 *t, int rows, __nv_b
     GemmArgs a{};
     a.work = c->work1; a.n_work = c->n_work; a.K = H; a.R = c->R1;
     a.n_kchunks = (H + kChunkK - 1) / kChunkK; a.n_ntiles = n_nt1;
-    a.w_tiles = w.w1_tiles; a.xq = c->xq; a.sfb = c->sfb_x; a.sfb_tile_stride = kSfbTileBytes; a.bias = w.b1; a.add_bias = 1;
+    a.w_tiles = w.w1_tiles; a.x_half0 = 0; a.sfb_tile0 = 0; a.sfb_step = 1; a.bias = w.b1; a.add_bias = 1;
     a.hq_out = c->hq; a.hq_joff = c->joff; a.hq_nkc = (c->Kw + kChunkK - 1) / kChunkK; a.y_out = nullptr; a.ld_out = c->Kw;
     a.h_exp = c->h_exp;
     a.limit = c->cfg.swiglu_limit; a.alpha = c->cfg.swiglu_alpha; a.status = status;
     GemmArgs b = a;
     b.work = c->work2; b.n_work = c->n_work + 1; b.K = c->Kw; b.R = H;
     b.n_kchunks = (c->Kw + kChunkK - 1) / kChunkK; b.n_ntiles = n_nt2;
-    b.w_tiles = w.w2_tiles; b.xq = c->hq; b.sfb = c->sfb_h; b.sfb_tile_stride = 0; b.bias = w.b2; b.add_bias = add_b2;
+    b.w_tiles = w.w2_tiles; b.x_half0 = c->max_tiles * slice_pairs(a.n_kchunks) * 2; b.sfb_tile0 = c->max_tiles; b.sfb_step = 0; b.bias = w.b2; b.add_bias = add_b2;
     b.hq_out = nullptr; b.y_out = c->ybuf; b.ld_out = H;
     MlpFuse fuse{};
     fuse.total_slot = c->max_tiles;
     fuse.done_per_tile = expert_mlp_done_per_tile(n_nt1);
     if (flags & MOE_FWD_SPLIT_MLP) {   // MLP1 and MLP2 as two launches
       fuse.phase_begin = 0; fuse.phase_end = 1; fuse.tile_done = nullptr;
-      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, fuse, c->gemm_grid, s, chained);
+      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, c->tm_x, fuse, c->gemm_grid, s, chained);
       mark();
       fuse.phase_begin = 1; fuse.phase_end = 2;
-      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, fuse, c->gemm_grid, s, chained);
+      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, c->tm_x, fuse, c->gemm_grid, s, chained);
     } else {                           // one launch; the MLP2 stage of a profile is then empty
       fuse.phase_begin = 0; fuse.phase_end = 2; fuse.tile_done = c->tile_done;
-      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, fuse, c->gemm_grid, s, chained);
+      launch_expert_mlp(w.tm_w1, a, w.tm_w2, b, c->tm_x, fuse, c->gemm_grid, s, chained);
       mark();
       c->launches -= 1;
       mlp_in_one_launch = true;
@@ -434,21 +460,21 @@ int moe_create(const moe_config *cfg, moe_handle *out) {
   const int n_kc1 = (c->H + kChunkK - 1) / kChunkK, n_kc2 = (c->Kw + kChunkK - 1) / kChunkK;
   const size_t xq_bytes = static_cast<size_t>(c->max_tiles) * slice_pairs(n_kc1) * kPairBytes;
   const size_t hq_bytes = static_cast<size_t>(c->max_tiles) * slice_pairs(n_kc2) * kPairBytes;
-  if ((rc = dev_alloc(c, &c->xq, xq_bytes))) return rc;
-  if ((rc = dev_alloc(c, &c->hq, hq_bytes))) return rc;
-  if ((rc = dev_alloc(c, &c->sfb_x, static_cast<size_t>(c->max_tiles) * kSfbTileBytes))) return rc;
-  if ((rc = dev_alloc(c, &c->sfb_h, static_cast<size_t>(kSfbTileBytes)))) return rc;
+  if ((rc = dev_alloc(c, &c->xq, xq_bytes + hq_bytes))) return rc;
+  c->hq = c->xq + xq_bytes;
+  const size_t sfb_bytes = static_cast<size_t>(c->max_tiles) * kSfbTileBytes;
+  if ((rc = dev_alloc(c, &c->sfb_x, sfb_bytes + kSfbTileBytes))) return rc;
   if ((rc = dev_alloc(c, &c->tile_base, static_cast<size_t>(c->E) + 1))) return rc;
-  CU_TRY(c, cudaMemset(c->xq, 0, xq_bytes));   // bytes past K in the last slice and never-written columns stay 0
-  CU_TRY(c, cudaMemset(c->hq, 0, hq_bytes));
-  CU_TRY(c, cudaMemset(c->sfb_x, 127, static_cast<size_t>(c->max_tiles) * kSfbTileBytes));
+  CU_TRY(c, cudaMemset(c->xq, 0, xq_bytes + hq_bytes));   // bytes past K in the last slice and never-written columns stay 0
+  CU_TRY(c, cudaMemset(c->sfb_x, 127, sfb_bytes));
   {
     uint8_t atoms[kSfbTileBytes];
     for (int r = 0; r < 256; ++r)
       for (int kb = 0; kb < 4; ++kb)
         atoms[r / 128 * kSfAtomBytes + (r % 32) * 16 + (r / 32 % 4) * 4 + kb] = static_cast<uint8_t>(127 + c->h_exp - ((r & 1) ? 4 : 0));
-    CU_TRY(c, cudaMemcpy(c->sfb_h, atoms, kSfbTileBytes, cudaMemcpyHostToDevice));
+    CU_TRY(c, cudaMemcpy(c->sfb_x + sfb_bytes, atoms, kSfbTileBytes, cudaMemcpyHostToDevice));
   }
+  if ((rc = make_token_maps(c, c->tm_x, c->xq, (xq_bytes + hq_bytes) / (kPairBytes / 2), c->sfb_x, static_cast<size_t>(c->max_tiles) + 1))) return rc;
   if ((rc = dev_alloc(c, &c->work1, (size_t)c->max_work1))) return rc;
   if ((rc = dev_alloc(c, &c->work2, (size_t)c->max_work2))) return rc;
   if ((rc = dev_alloc(c, &c->n_work, (size_t)2))) return rc;
@@ -486,7 +512,7 @@ int moe_destroy(moe_handle c) {
   cudaFree(c->offsets); cudaFree(c->pair_row); cudaFree(c->row_token); cudaFree(c->pair_slot); cudaFree(c->tile_done); cudaFree(c->xperm); cudaFree(c->hbuf);
   cudaFree(c->ybuf); cudaFree(c->out_f32); cudaFree(c->out_bf16); cudaFree(c->work1); cudaFree(c->work2);
   cudaFree(c->n_work); cudaFree(c->status);
-  cudaFree(c->xq); cudaFree(c->hq); cudaFree(c->sfb_x); cudaFree(c->sfb_h); cudaFree(c->tile_base);
+  cudaFree(c->xq); cudaFree(c->sfb_x); cudaFree(c->tile_base);
   delete c;
   return MOE_OK;
 }

@@ -128,9 +128,8 @@ struct GemmArgs {
   int n_kchunks;  // ceil(K / kChunkK)
   int n_ntiles;   // ceil(R / kBlockRows)
   const uint8_t *w_tiles;     // weight tiles [E][n_ntiles][2][n_kchunks * kWTileBytes], see LayerWeights::w1_tiles
-  const uint8_t *xq;          // token rows, e4m3 [tile][slice_pairs(n_kchunks)][kPairBytes] (x_pair_offset)
-  const uint8_t *sfb;         // their scales, kSfbTileBytes per token tile
-  int sfb_tile_stride;        // bytes between token tiles' scales (0: shared by all tiles)
+  int x_half0;                // token rows, e4m3 [tile][slice_pairs(n_kchunks)][2 halves]: the first half's place in TokenMaps
+  int sfb_tile0, sfb_step;    // their scales: place of tile 0 in TokenMaps, and of the next one (0: shared by all tiles)
   const __nv_bfloat16 *bias;  // [E][R]
   int add_bias;               // MLP2 on TP ranks other than 0 leaves the bias out
   uint8_t *hq_out;            // MLP1: quantised SwiGLU output, tiled like xq
@@ -152,6 +151,18 @@ struct MlpFuse {
   int done_per_tile;         // CTAs of a pair x MLP1 weight blocks
 };
 
+// Tensor maps of the quantised token rows, xq and hq as one array of halves (what one CTA of a pair reads of a pair of k
+// slices, kPairBytes / 2) and their scales as one array of kSfbTileBytes.  rows[g - 1]: a box is the first g 8-row groups
+// of both slices, 2 KB each, for tiles of tile_n = 16 g rows.
+struct TokenMaps {
+  CUtensorMap rows[kMaxTileTok / 8];
+  CUtensorMap scales;
+};
+// Tensor maps of a weight matrix: codes and scale atoms of a pair of k slices, and of the single last slice.
+struct WeightMaps {
+  CUtensorMap codes, scales, codes_last, scales_last;
+};
+
 struct LayerWeights {
   bool loaded = false;
   // MLP1 weights as the GEMM streams them, 8 KB per (expert, 240-row block, 120-row half, 128-wide slice of k):
@@ -167,7 +178,7 @@ struct LayerWeights {
   uint8_t *w2_scales_raw = nullptr;  // [E, H, Dl/32]
   __nv_bfloat16 *router_w3 = nullptr;  // [3][E][H] exact 3-way bf16 split of the fp32 router weight
   float *router_b = nullptr;           // [E]
-  CUtensorMap tm_w1[2], tm_w2[2];   // boxes of a pair of k slices, and of the single last one
+  WeightMaps tm_w1, tm_w2;
   CUtensorMap tm_router;
 };
 
@@ -205,9 +216,9 @@ struct moe_ctx {
   __half *xperm = nullptr;          // expert_input_buffer [max_pairs, H]   fp16 (validation GEMM only)
   __half *hbuf = nullptr;           // gate_up             [max_pairs, Dl]  fp16 (validation GEMM only)
   uint8_t *xq = nullptr;            // expert_input_buffer as e4m3 high/low rows, [max_tiles][pairs of k slices][kPairBytes]
-  uint8_t *hq = nullptr;            // gate_up as e4m3 high/low rows, same tiling over MLP2's k window
-  uint8_t *sfb_x = nullptr;         // per-tile scale atoms of xq [max_tiles][1024]
-  uint8_t *sfb_h = nullptr;         // the scale atoms of hq, the same for every tile [1024]
+  uint8_t *hq = nullptr;            // gate_up as e4m3 high/low rows, same tiling over MLP2's k window (behind xq, one allocation)
+  uint8_t *sfb_x = nullptr;         // per-tile scale atoms of xq [max_tiles][1024], then those of hq, the same for every tile
+  moe::TokenMaps tm_x;              // of xq, hq and their scales
   int *tile_base = nullptr;         // first token tile of each expert [E+1]
   int max_tiles = 0;
   int h_exp = 0;                    // hq holds e4m3(h * 2^-h_exp)
@@ -345,8 +356,8 @@ void launch_rmsnorm_rows(const __nv_bfloat16 *x, const __nv_bfloat16 *w, __nv_bf
 
 // expert_gemm_sm100.cu
 cudaError_t expert_gemm_init(int *grid);   // per-device kernel attributes; call with the device current
-void launch_expert_mlp(const CUtensorMap (&tm_w1)[2], const GemmArgs &a, const CUtensorMap (&tm_w2)[2], const GemmArgs &b,
-                       const MlpFuse &f, int grid, cudaStream_t s, bool chained);
+void launch_expert_mlp(const WeightMaps &tm_w1, const GemmArgs &a, const WeightMaps &tm_w2, const GemmArgs &b,
+                       const TokenMaps &tm_x, const MlpFuse &f, int grid, cudaStream_t s, bool chained);
 int expert_mlp_done_per_tile(int n_ntiles1);
 
 // tp_collectives.cu

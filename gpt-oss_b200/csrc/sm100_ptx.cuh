@@ -39,15 +39,16 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
 }
-// Arrives on the same barrier of CTA `cta` of the cluster.  Default semantics on purpose: what the arrival
-// publishes here are copies that the copy engine has completed and tensor-memory loads that have returned, no
-// ordinary stores of this thread, and a release at cluster scope is a memory barrier that costs ~0.9 us.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, uint32_t cta) {
-  asm volatile(
-      "{\n\t.reg .b32 r;\n\t"
-      "mapa.shared::cluster.u32 r, %0, %1;\n\t"
-      "mbarrier.arrive.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar), "r"(cta)
-      : "memory");
+// Address of the same place in CTA `cta` of the cluster.
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t cta) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(cta));
+  return r;
+}
+// Arrives on a barrier of any CTA of the cluster (bar: an address from map_to_cta), relaxed: for hand-overs of tensor
+// memory, whose accesses the tcgen05 fences on both sides order.  (Release at cluster scope is a memory barrier of ~0.9 us.)
+__device__ __forceinline__ void mbar_arrive_relaxed_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -58,15 +59,38 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// What a wait orders.  kCta: the default, acquire at CTA scope.  For barriers that another CTA of the cluster arrives on:
+// kCluster, acquire at cluster scope, for copies into shared memory; kClusterRelaxed, for hand-overs that need no data made
+// visible: tensor memory (the tcgen05 fences order it) and stages that the MMAs have finished reading.
+enum class Wait { kCta, kCluster, kClusterRelaxed };
+template <Wait kWait = Wait::kCta>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred P;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, P;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
+  if constexpr (kWait == Wait::kCluster) {
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  } else if constexpr (kWait == Wait::kClusterRelaxed) {
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 P, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  }
   return ok != 0;
 }
 // Bounded wait of a whole converged warp.  `abort_flag` is a CTA-shared word that any role sets when it
@@ -79,13 +103,14 @@ constexpr long long kWaitCycles = 2000000000LL;
 // operands of those instructions (descriptors, tensor-memory addresses) are then computed once per warp in
 // uniform registers; a lone diverged lane has to move every one of them there, which on this part costs
 // the issuing thread more than the instructions themselves.
+template <Wait kWait = Wait::kCta>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag,
                                                unsigned int *status, unsigned int code) {
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  if (__all_sync(0xffffffffu, mbar_try_wait<kWait>(bar, parity))) return true;
   const long long t0 = clock64();
   bool timed_out = false;
   for (uint32_t spin = 0;; ++spin) {
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if (__all_sync(0xffffffffu, mbar_try_wait<kWait>(bar, parity))) return true;
     if ((spin & 63u) == 63u) {
       timed_out = __any_sync(0xffffffffu, clock64() - t0 > kWaitCycles);
       if (timed_out || __any_sync(0xffffffffu, *abort_flag != 0u)) break;
@@ -124,39 +149,49 @@ __device__ __forceinline__ uint64_t l2_policy_evict_first() {
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
-__device__ __forceinline__ void tma_load_3d_hint(uint32_t dst, const CUtensorMap *m, int x, int y, int z, uint32_t bar,
-                                                 uint64_t policy) {
+// Loads of a CTA pair: into this CTA's shared memory, completion on a barrier of either CTA of the pair (bar: an address
+// from map_to_cta).  The copy engine's completion has release semantics at cluster scope.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *m, int x, int y, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint"
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
+      " [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap *m, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
+      " [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair_hint(uint32_t dst, const CUtensorMap *m, int x, int y, uint32_t bar,
+                                                      uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2.L2::cache_hint"
+      " [%0], [%1, {%3, %4}], [%2], %5;"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y), "l"(policy)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair_hint(uint32_t dst, const CUtensorMap *m, int x, int y, int z, uint32_t bar,
+                                                      uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2.L2::cache_hint"
       " [%0], [%1, {%3, %4, %5}], [%2], %6;"
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y), "r"(z), "l"(policy)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_5d_hint(uint32_t dst, const CUtensorMap *m, int x, int y, int z, int u, int v,
-                                                 uint32_t bar, uint64_t policy) {
+__device__ __forceinline__ void tma_load_5d_pair_hint(uint32_t dst, const CUtensorMap *m, int x, int y, int z, int u, int v, uint32_t bar,
+                                                      uint64_t policy) {
   asm volatile(
-      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint"
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2.L2::cache_hint"
       " [%0], [%1, {%3, %4, %5, %6, %7}], [%2], %8;"
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(u), "r"(v), "l"(policy)
-      : "memory");
-}
-__device__ __forceinline__ void bulk_load_hint(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar,
-                                               uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar), "l"(policy)
       : "memory");
 }
 // Brings `bytes` (a multiple of 16, 16-byte aligned) into L2.
 __device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<uint64_t>(src)), "r"(bytes) : "memory");
-}
-// Untiled bulk copy: both addresses 16-byte aligned, size a multiple of 16.
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
-      : "memory");
 }
 
 // ---------------------------------------------------------------- tensor memory

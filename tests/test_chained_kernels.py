@@ -6,7 +6,10 @@ other kernels are still writing, so none of it may come through the read-only pa
 anything but a layer's constants.
 
 The warp that counts finished MLP1 items publishes rows that sixteen other warps wrote: acquire in every lane, warp
-barrier, fence in every lane, then the counts."""
+barrier, fence in every lane, then the counts.
+
+What one CTA of a pair hands to the other needs cluster scope: copies complete on the even CTA's barrier by themselves,
+and arrivals there name their scope."""
 import glob
 import os
 import re
@@ -47,10 +50,21 @@ def test_no_bounded_wait_starts_before_the_predecessor_is_done():
     bounded waits passes the grid wait first."""
     body = {n: b for n, _, b in kernels()}
     gemm = body["expert_gemm_kernel"]
-    assert gemm.index("grid_dep_sync();") < gemm.index("mbar_wait_warp(")
+    assert gemm.index("grid_dep_sync();") < gemm.index("mbar_wait_warp")
     router = body["router_kernel"]
     roles = re.split(r"(?:if|else if) \(warp (?:==|<) \d\) \{", router[router.index("grid_dep_release();"):])
-    roles = [r for r in roles[1:] if "mbar_wait_warp(" in r]
+    roles = [r for r in roles[1:] if "mbar_wait_warp" in r]
     assert len(roles) == 3
     for r in roles:
-        assert "grid_dep_wait();" in r and r.index("grid_dep_wait();") < r.index("mbar_wait_warp(")
+        assert "grid_dep_wait();" in r and r.index("grid_dep_wait();") < r.index("mbar_wait_warp")
+
+
+def test_hand_overs_of_a_cta_pair_have_cluster_scope():
+    body = {n: b for n, _, b in kernels()}["expert_gemm_kernel"]
+    ptx = open(os.path.join(ROOT, "gpt-oss_b200", "csrc", "sm100_ptx.cuh")).read()
+    for arrive in re.findall(r"mbarrier\.arrive[\w.:]*shared::cluster", ptx):
+        assert ".cluster.shared::cluster" in arrive, arrive
+    assert not re.search(r"\b(tma_load_\dd|tma_load_\dd_hint|bulk_load\w*)\(", body)    # only loads of the pair
+    waits = re.findall(r"mbar_wait_warp(<Wait::k(?:Cluster|ClusterRelaxed)>)?\((\w+)_bar", body)
+    assert {bar for _, bar in waits} == {"full", "empty", "dfull", "dempty"}
+    assert all(scope for scope, _ in waits) and ("<Wait::kCluster>", "full") in waits
