@@ -447,7 +447,7 @@ int moe_create(const moe_config *cfg, moe_handle *out) {
   CU_TRY(c, cudaEventCreateWithFlags(&c->ev_fork2, cudaEventDisableTiming));
   CU_TRY(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
   const int n_nt1 = (c->R1 + kBlockRows - 1) / kBlockRows, n_nt2 = (c->H + kBlockRows - 1) / kBlockRows;
-  c->max_tiles = c->max_pairs / kMaxTileTok + c->E + 1;
+  c->max_tiles = max_token_tiles(c->max_pairs, c->E);
   if ((rc = dev_alloc(c, &c->tile_done, static_cast<size_t>(c->max_tiles) + 1))) return rc;
   c->max_work1 = c->max_tiles * n_nt1;
   c->max_work2 = c->max_tiles * n_nt2;

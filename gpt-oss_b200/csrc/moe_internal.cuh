@@ -37,6 +37,12 @@ __host__ __device__ inline int tokens_per_tile(int cnt) {
   const int n = expert_tiles(cnt);
   return n == 0 ? kMaxTileTok : ((cnt + n - 1) / n + 7) / 8 * 8;
 }
+// Most tiles that `pairs` (token, expert) pairs over E experts can need: ceil(cnt / max) is at most 1 + (cnt - 1) / max for
+// each expert with rows, and there are at most min(E, pairs) of those.  (All experts get 97 rows: exactly this many.)
+inline int max_token_tiles(int pairs, int E) {
+  const int experts = std::min(pairs, E);
+  return experts + (pairs - experts) / kMaxTileTok;
+}
 __host__ __device__ inline int slice_pairs(int n_slices) { return (n_slices + 1) / 2; }
 
 // Token rows of a tile: [pair of k slices][CTA][8-row group][slice of the pair][8 rows][128 bytes].  Four tokens make

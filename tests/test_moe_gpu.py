@@ -170,6 +170,19 @@ def test_routing_invariants(pkg, synth):
         blk.close()
 
 
+def test_a_handle_for_one_row_is_small(pkg):
+    """The quantised rows are laid out in tiles of 96 tokens; a handle has as many as its rows can need (here four, 4.7 MB
+    for both GEMMs), not one for every expert (151 MB)."""
+    import torch
+    torch.zeros(1, device="cuda")
+    free = torch.cuda.mem_get_info()[0]
+    blk = pkg.MoeBlock(2880, 2880, 128, max_rows=1)
+    try:
+        assert free - torch.cuda.mem_get_info()[0] < 64 << 20
+    finally:
+        blk.close()
+
+
 @pytest.mark.parametrize("top_k", [3, 4])
 @pytest.mark.parametrize("T", [511, 512, 513, 2047, 2048, 2049, 8192, 8225])
 def test_index_at_the_edges_of_its_forms(T, top_k, pkg, synth):
