@@ -47,8 +47,10 @@
 // Measured (B200, one launch of both phases, us, layer of 128 experts, hidden and intermediate size 2880; before: one CTA
 // per item of 64 tokens x 240 rows, tokens on the fixed M = 128 axis), without the L2 prefetch further down: 32 rows
 // 179 -> 174, 256 rows 324 -> 299, 1856 rows 412 -> 396, 8192 rows 1459 -> 1403.  Bound by HBM up to ~16 tokens per
-// expert, by the shared-memory port around 60 (712 of 773 cycles per stage), by the tensor pipe above (86 % of the cycles
-// at 8192 rows, where the power cap sets the clock to 1.29 GHz).
+// expert, by the tensor pipe at 8192 rows (86 % of the cycles, at the 1.29 GHz that the power cap leaves).  In between no
+// single bound is shown: at 1856 rows (~58 tokens per expert) a stage takes 773 cycles, the tensor pipe 492 of them and HBM
+// ~550.  A count of all bytes through the shared-memory port at 128 a cycle gives 734, but the same count at 8192 rows
+// asks for more than what is measured there (~420 against 388 cycles per slice), so the port is not it as counted.
 #include <cuda_fp8.h>
 
 #include "moe_internal.cuh"

@@ -374,8 +374,8 @@ quantize_few_rows_kernel(const __nv_bfloat16 *t, const int2 *pair_slot, int T, i
   for (int k = 0; k < kSlots; ++k) slot[k] = k < K ? pair_slot[static_cast<size_t>(tok) * K + k] : make_int2(-1, 0);
   const uint4 *src = reinterpret_cast<const uint4 *>(t + static_cast<size_t>(tok) * H);
   const int ngrp = H / 16;    // a lane takes groups of 16 elements: 32 bytes in, 16 + 16 bytes out
-  // Largest magnitude: bf16 magnitudes compare like their bit patterns.  (A NaN wins, and every output of its token is
-  // NaN whatever the scale.)
+  // Largest magnitude: bf16 magnitudes compare like their bit patterns.  (A NaN wins.  Whatever the scale, all of its
+  // token's MLP1 sums are then NaN, which the SwiGLU's clamps turn into their limits.)
   uint32_t top = 0;
 #pragma unroll 6
   for (int g = lane; g < ngrp; g += 32) {
