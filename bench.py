@@ -59,7 +59,7 @@ CPU_SAMPLE_TOKENS = 32
 PARITY_ROWS = 64
 # dram read+write bytes / algorithmic bytes of the expert MLP kernel, from an ncu capture of a 4x smaller case
 # (20B shape, 464 rows: the same rows per expert); traffic is proportional to the weights streamed
-NCU_TRAFFIC_PER_ALGORITHMIC_BYTE = 1.039
+NCU_TRAFFIC_PER_ALGORITHMIC_BYTE = 1.041
 
 
 def tp_size_for(n_gpus: int, parallel: str, tp_arg: int) -> int:
