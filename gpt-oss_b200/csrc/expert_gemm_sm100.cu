@@ -35,9 +35,9 @@
 // instructions per slice for the pair.  The copies of both CTAs complete on the even CTA's barrier (loads of
 // cta_group::2, whose completion is a release at cluster scope), where its MMA warp acquires them at cluster scope.
 // (The odd CTA used to report what had landed with an arrival of CTA scope, which promises nothing across CTAs; with
-// release at cluster scope such a report costs 0.9 us a stage.  Whole calls, us, report of CTA scope / now / now but with
-// the acquire left out: 1 row 39.4 / 39.2 / 39.0, 32 rows 185.2 / 186.2 / 184.5, 64 rows of 32 experts 102.9 / 103.9 /
-// 103.1, 256 rows (block) 330 / 332 / 330, larger ones within the spread of the runs.)
+// release at cluster scope such a report costs 0.9 us a stage.  Whole calls, us, report of CTA scope / now: 1 row 39.3 /
+// 39.0, 32 rows 185.8 / 185.9, 64 rows of 32 experts 102.8 / 103.1, 256 rows (block) 330 / 331, larger ones within the spread
+// of the runs.)
 // Issuing warps stay converged and elect one lane, so that descriptors and
 // tensor-memory addresses live in uniform registers.  Sixteen epilogue warps per CTA drain the
 // fp32 accumulator (double buffered: 2 x 192 columns).

@@ -60,21 +60,15 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // What a wait orders.  kCta: the default, acquire at CTA scope.  For barriers that another CTA of the cluster arrives on:
-// kCluster, acquire at cluster scope, for copies into shared memory; kClusterRelaxed, for hand-overs that need no data made
-// visible: tensor memory (the tcgen05 fences order it) and stages that the MMAs have finished reading.
+// kCluster, acquire at cluster scope of what lies in the cluster's shared memory, for copies into it; kClusterRelaxed, for
+// hand-overs that need no data made visible: tensor memory (the tcgen05 fences order it) and stages that the MMAs have
+// finished reading.  The acquire is a fence behind a relaxed wait: an acquire of all memory in the wait itself, polls
+// included, cost 1 % of a small call.
 enum class Wait { kCta, kCluster, kClusterRelaxed };
 template <Wait kWait = Wait::kCta>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  if constexpr (kWait == Wait::kCluster) {
-    asm volatile(
-        "{\n\t.reg .pred P;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, P;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-  } else if constexpr (kWait == Wait::kClusterRelaxed) {
+  if constexpr (kWait != Wait::kCta) {
     asm volatile(
         "{\n\t.reg .pred P;\n\t"
         "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 P, [%1], %2;\n\t"
@@ -106,11 +100,16 @@ constexpr long long kWaitCycles = 2000000000LL;
 template <Wait kWait = Wait::kCta>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag,
                                                unsigned int *status, unsigned int code) {
-  if (__all_sync(0xffffffffu, mbar_try_wait<kWait>(bar, parity))) return true;
+  auto passed = [&]() -> bool {
+    if (!__all_sync(0xffffffffu, mbar_try_wait<kWait>(bar, parity))) return false;
+    if constexpr (kWait == Wait::kCluster) asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+    return true;
+  };
+  if (passed()) return true;
   const long long t0 = clock64();
   bool timed_out = false;
   for (uint32_t spin = 0;; ++spin) {
-    if (__all_sync(0xffffffffu, mbar_try_wait<kWait>(bar, parity))) return true;
+    if (passed()) return true;
     if ((spin & 63u) == 63u) {
       timed_out = __any_sync(0xffffffffu, clock64() - t0 > kWaitCycles);
       if (timed_out || __any_sync(0xffffffffu, *abort_flag != 0u)) break;

@@ -68,3 +68,4 @@ def test_hand_overs_of_a_cta_pair_have_cluster_scope():
     waits = re.findall(r"mbar_wait_warp(<Wait::k(?:Cluster|ClusterRelaxed)>)?\((\w+)_bar", body)
     assert {bar for _, bar in waits} == {"full", "empty", "dfull", "dempty"}
     assert all(scope for scope, _ in waits) and ("<Wait::kCluster>", "full") in waits
+    assert "fence.acquire.sync_restrict::shared::cluster.cluster" in ptx
