@@ -190,8 +190,8 @@ expert_gemm_kernel(const __grid_constant__ WeightMaps tm_w1, const __grid_consta
   };
   unsigned int *status = pa.status;
   bool ok = true;
-  // The even CTA's full barriers.  A copy of the odd CTA for the next round of a stage cannot come early: it waits for the
-  // MMAs of this round, which wait for the barrier's phase.
+  // The even CTA's full barriers.  A copy of the odd CTA for the next use of a stage cannot come early: it waits for the
+  // MMAs of the present one, which wait for the barrier's phase.
   const uint32_t full0 = map_to_cta(full_bar(0), 0);
 
   if (warp == kWProducerWarp) {
